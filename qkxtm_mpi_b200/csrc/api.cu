@@ -13,8 +13,8 @@
 
 #include "blas.cuh"
 #include "hop.cuh"
-#include "hop_c3.cuh"
 #include "hop_c3t.cuh"
+#include "hop_s2.cuh"
 #include "layout.cuh"
 #include "qkx_ctx.cuh"
 #include "site_ops.cuh"
@@ -138,9 +138,6 @@ static double hop_bytes(size_t nout, double S, double G, bool both, bool extra_x
   return (double)nout * (2 * S + (both ? 4 : 8) * G + (extra_x ? S : 0));
 }
 
-// FP64 sites per block of the colour-split kernel (x 3 colour threads)
-constexpr int C3_NS = 64;
-
 // cuTensorMapEncodeTiled of the driver, looked up once (the library links the runtime only)
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -216,8 +213,19 @@ static bool launch_hop64_tiled(qkx_ctx* c, HopArgs<SpinorF64, GaugeF64x18>& A, c
 template <int B, bool DAG, int EPI>
 static int launch_hop64(qkx_ctx* c, HopArgs<SpinorF64, GaugeF64x18>& A, const HopRes& Rz = HopRes{}) {
   if (launch_hop64_tiled<B, DAG, EPI>(c, A, Rz)) return QKX_OK;
-  A.nblk = c3_blocks_per_rhs<C3_NS>(c->Vh, A.out_parity);
-  hop_c3_kernel<C3_NS, SpinorF64, B, DAG, EPI><<<A.nblk * A.nrhs, dim3(C3_NS, 3), 0, c->st>>>(A, Rz);
+  A.nblk = s2_blocks_per_rhs(c->Vh, A.out_parity);
+  // Two right-hand sides a thread share the link loads (2.60 -> 2.36 ms for 12 at 32^3x64), as long as
+  // the halved grid still fills the SMs at its 6 blocks each; below that (8^3x16 with 12: 128 site
+  // blocks) one a thread keeps more SMs busy.  Only the batches (UKQCD, D) come with nrhs > 1.
+  if constexpr (B == 0 && !DAG) {
+    const int ngrp = (A.nrhs + 1) / 2;
+    if (A.nrhs > 1 && A.nblk * ngrp >= 148 * 6) {
+      hop_s2_kernel<2, B, DAG, EPI><<<A.nblk * ngrp, 2 * S2_NS, 0, c->st>>>(A, Rz);
+      counted(c);
+      return QKX_OK;
+    }
+  }
+  hop_s2_kernel<1, B, DAG, EPI><<<A.nblk * A.nrhs, 2 * S2_NS, 0, c->st>>>(A, Rz);
   counted(c);
   return QKX_OK;
 }

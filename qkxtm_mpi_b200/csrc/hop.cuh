@@ -28,13 +28,13 @@ enum Epilogue {
   EPI_XPAY_G5 = 2,     // out = g5 (a D psi + x + i c g5 x)      (normal operator through the g5 trick)
   EPI_TWIST_INV = 3,   // out = s (v - i c g5 v), v = D psi      (A^-1 D, first step of tm_xx)
   EPI_XPAY_TWINV = 4,  // out = s (v - i c g5 v), v = a D psi + x (odd-parity reconstruction)
-  EPI_XPAY_G5_RES = 5, // res = w - g5 (a D psi + x + i c g5 x), stored in FP32 (hop_c3_kernel only)
-  EPI_XPAY_RES = 6,    // res = w - (a D psi + x + i c g5 x), its norm only (hop_c3_kernel only)
+  EPI_XPAY_G5_RES = 5, // res = w - g5 (a D psi + x + i c g5 x), stored in FP32 (hop_s2_kernel and hop_c3t_kernel)
+  EPI_XPAY_RES = 6,    // res = w - (a D psi + x + i c g5 x), its norm only (hop_s2_kernel and hop_c3t_kernel)
   EPI_XPAY_G5_CGR = 7, // o = g5 (a D psi + x + i c g5 x) is not stored: the CG residual of the batch
                        // takes it, r -= alpha o, and |r|^2 goes to the norm partials (multi-RHS
                        // kernels of the mixed solver only; r is racc32, or racc64 for FP64 sloppy)
   EPI_XPAY_TWINV_RES = 8,  // as EPI_XPAY_TWINV, and |v - (out + i c g5 out)|^2 to the norm partials: with
-                           // x = b_o, a = kappa the odd half of ||b - M x||^2 (hop_c3_kernel only)
+                           // x = b_o, a = kappa the odd half of ||b - M x||^2 (the same)
 };
 
 // extra operands of EPI_XPAY_G5_RES / EPI_XPAY_RES: w, and the FP32 field the residual

@@ -1,12 +1,11 @@
 // hop_c3t.cuh -- the FP64 hopping term on row tiles that TMA stages in shared
 // memory.
 //
-// Same operator, colour split and epilogues as hop_c3_kernel (reference
+// Same operator and epilogues as hop_s2_kernel, split by colour (reference
 // Vector::applyDslash / applyDslashDag, lib/lattice_util.cpp:1158-1213,
 // 1643-1699; 18-real links as given), different data movement.  The direct
-// kernel issues, per colour thread and neighbour term, fifteen 16-byte global
-// loads at computed 64-bit addresses; half of its instructions are those loads
-// and their address arithmetic, and each neighbour spinor is fetched from L2 by
+// kernel issues, per thread and neighbour term, fifteen 16-byte global loads at
+// computed 64-bit addresses, and each neighbour spinor is fetched from L2 by
 // up to eight sites.  Here a block owns a tile of C3T_ROWS consecutive lattice
 // rows (fixed z, t, one output parity): W = L0/2 sites a row, 4W sites, three
 // colour threads each.  Every input the tile needs is a few contiguous site
@@ -35,7 +34,7 @@
 // block (six warps) runs on an SM.  Those six warps cannot hide the latency of
 // the FP64 arithmetic and shared-memory reads, and with one right-hand side
 // nothing overlaps a tile's staging with its compute (32^3x64 tm: 1.11 ms
-// against 0.61 ms a launch; the 12-RHS reliable-update hops lose too).
+// against 0.47 ms a launch; the 12-RHS reliable-update hops lose too).
 #pragma once
 #include <cuda.h>
 
