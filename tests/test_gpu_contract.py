@@ -96,3 +96,21 @@ def test_argument_checks(qkx):
             lat.delta_2pt(p, p, 2)
         with pytest.raises(qkx.QkxError):
             lat.meson_2pt(p, [0], Q_sq=-1)
+
+
+@pytest.mark.parametrize("L,Q", [((2, 3, 3, 5), 2), ((2, 2, 2, 2), 0), ((14, 3, 5, 2), 9)])
+def test_partial_site_blocks_and_momentum_chunks(qkx, oracle, L, Q):
+    """V = 90, 16 and 420: remainders of the 8-site blocks; 1 to 29 distinct (p_x, p_y), i.e. partial
+    chunks of the transform; every operator, one propagator standing for both as well."""
+    p1, p2 = seeded_propagator(L, 11 + L[0]), seeded_propagator(L, 12 + L[0])
+    xs = (1, 1, 1, 1)
+    with qkx.Lattice(qkx.LatticeInfo(L=L)) as lat:
+        m = lat.meson_2pt(p1, range(10), Q, xs)
+        for op in range(10):
+            assert _close(m[op], oracle.meson_2pt(L, p1, op, Q, xs)), op
+        for op in range(4):
+            assert _close(lat.baryon_2pt(p1, p2, op, Q, xs), oracle.baryon_2pt(L, p1, p2, op, Q, xs)), op
+        assert _close(lat.baryon_2pt(p2, p2, 0, Q, xs), oracle.baryon_2pt(L, p2, p2, 0, Q, xs))
+        if Q < 9:
+            for op in range(2):
+                assert _close(lat.delta_2pt(p1, p2, op, Q, xs), oracle.delta_2pt(L, p1, p2, op, Q, xs)), op
