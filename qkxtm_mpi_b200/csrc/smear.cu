@@ -117,77 +117,24 @@ int ape_run(qkx_ctx* c, const double2* in, double2* R, double2* T, int nsmear, d
 }
 
 // ---------------------------------------------------------------- Gaussian smearing
-struct GaussTile {
-  int nr, nt;
-};
-constexpr GaussTile kGaussTiles[] = {{1, 64}, {1, 128}, {1, 256}, {2, 64}, {2, 128}, {2, 256}};
-
-template <int NT, int NR>
+template <int NSP, int NR>
 void launch_gauss_t(qkx_ctx* c, const FieldPtrs& in, const FieldPtrs& out, int nrhs, int cb0, int ncb, double alpha,
                     double norm) {
-  const int nblk = (ncb + NT - 1) / NT;
+  const int nblk = (ncb + 31) / 32;
   const int ngrp = (nrhs + NR - 1) / NR;
-  k_gauss_step<NT, NR><<<(unsigned)nblk * 2 * ngrp, NT, 0, c->st>>>(in, out, GaugeF64x18{c->Usm, c->Vh}, c->geom,
-                                                                     nrhs, cb0, ncb, alpha, norm);
+  k_gauss_step<NSP, NR><<<(unsigned)nblk * 2 * ngrp, 32 * 4 / NSP, 0, c->st>>>(in, out, GaugeF64x18{c->Usm, c->Vh},
+                                                                              c->geom, nrhs, cb0, ncb, alpha, norm);
 }
 
-int launch_gauss(qkx_ctx* c, GaussTile t, const FieldPtrs& in, const FieldPtrs& out, int nrhs, int cb0, int ncb,
-                 double alpha, double norm) {
-  switch (t.nr * 1000 + t.nt) {
-    case 1064: launch_gauss_t<64, 1>(c, in, out, nrhs, cb0, ncb, alpha, norm); break;
-    case 1128: launch_gauss_t<128, 1>(c, in, out, nrhs, cb0, ncb, alpha, norm); break;
-    case 1256: launch_gauss_t<256, 1>(c, in, out, nrhs, cb0, ncb, alpha, norm); break;
-    case 2064: launch_gauss_t<64, 2>(c, in, out, nrhs, cb0, ncb, alpha, norm); break;
-    case 2128: launch_gauss_t<128, 2>(c, in, out, nrhs, cb0, ncb, alpha, norm); break;
-    case 2256: launch_gauss_t<256, 2>(c, in, out, nrhs, cb0, ncb, alpha, norm); break;
-    default: set_error("internal: no smearing tile %d/%d", t.nr, t.nt); return QKX_ERR_INVALID;
-  }
+// Four colour vectors a loaded link is the best use of the registers (times at the kernel): one spin of 4
+// fields, or of 3 where that leaves fewer spare slots (3, 5, 6, 9 fields), or two spins of 1 field for 1 or 2.
+int launch_gauss(qkx_ctx* c, const FieldPtrs& in, const FieldPtrs& out, int nrhs, int cb0, int ncb, double alpha,
+                 double norm) {
+  if (nrhs <= 2) launch_gauss_t<2, 1>(c, in, out, nrhs, cb0, ncb, alpha, norm);
+  else if ((nrhs + 2) / 3 * 3 - nrhs < (nrhs + 3) / 4 * 4 - nrhs) launch_gauss_t<1, 3>(c, in, out, nrhs, cb0, ncb, alpha, norm);
+  else launch_gauss_t<1, 4>(c, in, out, nrhs, cb0, ncb, alpha, norm);
   counted(c);
   QKX_CUDA(cudaGetLastError());
-  return QKX_OK;
-}
-
-// The tile (right-hand sides per thread, threads per block) of the smearing
-// step for a batch size, timed once per context on a full-lattice step from
-// `in` into `scratch` (the caller's data are not changed).
-int gauss_tile(qkx_ctx* c, int nrhs, const FieldPtrs& in, const FieldPtrs& scratch, double alpha, double norm,
-               GaussTile* out) {
-  const int key = 900000 + nrhs;
-  auto it = c->tuned.find(key);
-  if (it != c->tuned.end()) {
-    *out = {it->second.nr, it->second.nt};
-    return QKX_OK;
-  }
-  cudaEvent_t a, b;
-  QKX_CUDA(cudaEventCreate(&a));
-  QKX_CUDA(cudaEventCreate(&b));
-  GaussTile best = kGaussTiles[0];
-  float best_ms = 1e30f;
-  int rc = QKX_OK;
-  for (const GaussTile& t : kGaussTiles) {
-    if (t.nr > 1 && nrhs < t.nr) continue;
-    float ms = 0;
-    for (int rep = 0; rep < 3 && rc == QKX_OK; rep++) {  // first run warms up
-      if (cudaEventRecord(a, c->st) != cudaSuccess) rc = QKX_ERR_CUDA;
-      if (rc == QKX_OK) rc = launch_gauss(c, t, in, scratch, nrhs, 0, c->Vh, alpha, norm);
-      if (rc == QKX_OK && cudaEventRecord(b, c->st) != cudaSuccess) rc = QKX_ERR_CUDA;
-      if (rc == QKX_OK && cudaEventSynchronize(b) != cudaSuccess) rc = QKX_ERR_CUDA;
-      float m = 0;
-      if (rc == QKX_OK && cudaEventElapsedTime(&m, a, b) != cudaSuccess) rc = QKX_ERR_CUDA;
-      if (rep > 0) ms += m;
-    }
-    if (rc != QKX_OK) break;
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = t;
-    }
-  }
-  cudaEventDestroy(a);
-  cudaEventDestroy(b);
-  if (rc == QKX_ERR_CUDA) set_error("smearing tile timing: %s", cudaGetErrorString(cudaGetLastError()));
-  if (rc != QKX_OK) return rc;
-  c->tuned[key] = {best.nr, best.nt, 0};
-  *out = best;
   return QKX_OK;
 }
 
@@ -198,14 +145,12 @@ int gauss_tile(qkx_ctx* c, int nrhs, const FieldPtrs& in, const FieldPtrs& scrat
 int gauss_run(qkx_ctx* c, int nrhs, const FieldPtrs& in, const FieldPtrs& out, const FieldPtrs& tmp, int nsmear,
               double alpha, int cb0, int ncb) {
   const double norm = 1.0 / (1.0 + 6.0 * alpha);
-  GaussTile tile;
-  QKX_TRY(gauss_tile(c, nrhs, in, tmp, alpha, norm, &tile));
   const double bytes = 2.0 * ncb * (384.0 * nrhs + 432.0);
   const FieldPtrs* src = &in;
   const FieldPtrs* dst = (nsmear & 1) ? &out : &tmp;
   for (int it = 0; it < nsmear; it++) {
     QKX_TRY(prof_begin(c));
-    QKX_TRY(launch_gauss(c, tile, *src, *dst, nrhs, cb0, ncb, alpha, norm));
+    QKX_TRY(launch_gauss(c, *src, *dst, nrhs, cb0, ncb, alpha, norm));
     QKX_TRY(prof_end(c, bytes));
     src = dst;
     dst = (dst == &out) ? &tmp : &out;

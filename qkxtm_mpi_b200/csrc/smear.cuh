@@ -297,91 +297,101 @@ struct FieldPtrs {
   const double2* p[MAX_RHS];
 };
 
-__device__ __forceinline__ void load_sp(const double2* f, int Vh, int parity, int cb, Spinor<double>& s) {
-  const double2* b = f + (size_t)parity * 12 * Vh + cb;
-#pragma unroll
-  for (int k = 0; k < 12; k++) {
-    const double2 d = __ldg(b + (size_t)k * Vh);
-    s.c[k / 3][k % 3] = {d.x, d.y};
-  }
-}
-
-// acc += U v (dag = false) or U^dag v (dag = true), on all four spins
+// acc += U v (DAG false) or U^+ v (DAG true) on one spin, in FMA chains
 template <bool DAG>
-__device__ __forceinline__ void link_spinor_acc(const Lk& u, const Spinor<double>& v, Spinor<double>& acc) {
+__device__ __forceinline__ void link_vec_acc(const Cd (&u)[9], const Cd (&v)[3], Cd (&acc)[3]) {
 #pragma unroll
-  for (int s = 0; s < 4; s++)
+  for (int a = 0; a < 3; a++)
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-      Cd t = acc.c[s][a];
-#pragma unroll
-      for (int b = 0; b < 3; b++) t = t + (DAG ? cmulc(u.m[b][a], v.c[s][b]) : cmul(u.m[a][b], v.c[s][b]));
-      acc.c[s][a] = t;
+    for (int b = 0; b < 3; b++) {
+      const Cd e = DAG ? conj(u[b * 3 + a]) : u[a * 3 + b];
+      acc[a].re = fma(e.re, v[b].re, acc[a].re);
+      acc[a].im = fma(e.re, v[b].im, acc[a].im);
+      acc[a].re = fma(-e.im, v[b].im, acc[a].re);
+      acc[a].im = fma(e.im, v[b].re, acc[a].im);
     }
 }
 
 // One smearing iteration on sites cb in [cb0, cb0 + ncb) of both parities:
 //   out = norm * (in + alpha * sum_{mu<3} [U_mu(x) in(x+mu) + U_mu(x-mu)^dag in(x-mu)])
-// Each thread takes one site for NR right-hand sides, so every link is loaded
-// once per NR fields.  blockIdx.x = ((block * 2) + parity) * ngroups + group,
-// the groups of one site block adjacent so their shared links stay in L2.
-template <int NT, int NR>
-__global__ void __launch_bounds__(NT) k_gauss_step(FieldPtrs in, FieldPtrs out, GaugeF64x18 u, Geom g, int nrhs,
-                                                   int cb0, int ncb, double alpha, double norm) {
+// The stencil acts on every spin alike, so a site is split over 4/NSP threads of NSP spins each, and
+// a thread takes NR right-hand sides: a loaded link serves NSP * NR colour vectors.  A block covers
+// 32 sites with one warp per spin group (the warps share the links through L1).
+// blockIdx.x = ((block * 2) + parity) * ngroups + group, the groups of one site block adjacent so
+// their shared links stay in L2.
+//
+// What bounds it: the L1 data path (65% busy) and the latency of the gathers at 16 warps an SM; the FP64 pipe
+// is 38% busy.  Per step on one B200, against a whole site and two fields a thread (255 registers, 8 warps):
+//   24^3x48, 12 fields (NSP 1, NR 4)   1.29 -> 1.11 ms        16^3x32, 3 fields (1, 3)   0.074 -> 0.064 ms
+//   24^3x48,  1 field  (NSP 2, NR 1)   0.137 -> 0.120 ms      8x6x10x12, 5 fields        10.4 -> 8-10 us
+// Slower at 12 fields: (1, 1) 1.73, (1, 2) 1.36, (1, 3) 1.15, (1, 6) 1.21, (2, 1) 1.19, (2, 2) 1.21, (2, 3) 1.14 ms,
+// and 168 registers at 12 warps for any of them.
+template <int NSP, int NR>
+__global__ void __launch_bounds__(32 * 4 / NSP, 4 * NSP)
+    k_gauss_step(FieldPtrs in, FieldPtrs out, GaugeF64x18 u, Geom g, int nrhs, int cb0, int ncb, double alpha,
+                 double norm) {
   const int ngrp = (nrhs + NR - 1) / NR;
-  const int grp = blockIdx.x % ngrp;
+  const int r0 = (blockIdx.x % ngrp) * NR;
   const int bp = blockIdx.x / ngrp;
   const int par = bp & 1;
-  const int i = (bp >> 1) * NT + threadIdx.x;
+  const int i = (bp >> 1) * 32 + (threadIdx.x & 31);
   if (i >= ncb) return;
-  const int cb = cb0 + i;
-  const int r0 = grp * NR;
+  const int cb = cb0 + i, s0 = (threadIdx.x >> 5) * NSP;
   int x[4];
   cb_coords(g, cb, par, x);
   const int L0 = g.L[0], L01 = L0 * g.L[1];
   const int s = x[0] + L0 * x[1] + L01 * x[2] + L01 * g.L[2] * x[3];
   const int Vh = g.Vh;
-  Spinor<double> acc[NR];
+  // a group's spare slots read its last field and store nothing
+  const double2* f[NR];
+#pragma unroll
+  for (int j = 0; j < NR; j++) f[j] = in.p[min(r0 + j, nrhs - 1)] + (size_t)(s0 * 3) * Vh;
+  Cd acc[NR][NSP][3];
 #pragma unroll
   for (int j = 0; j < NR; j++)
 #pragma unroll
-    for (int k = 0; k < 12; k++) acc[j].c[k / 3][k % 3] = {0.0, 0.0};
+    for (int k = 0; k < NSP; k++)
+#pragma unroll
+      for (int a = 0; a < 3; a++) acc[j][k][a] = {0.0, 0.0};
 #pragma unroll
   for (int mu = 0; mu < 3; mu++) {
     const int stride = mu == 0 ? 1 : (mu == 1 ? L0 : L01);
     const int Lm = g.L[mu];
     const int nf = (x[mu] == Lm - 1 ? s - (Lm - 1) * stride : s + stride) >> 1;
     const int nb = (x[mu] == 0 ? s + (Lm - 1) * stride : s - stride) >> 1;
-    {
-      const Lk uf = u.load(par, mu, cb);
 #pragma unroll
-      for (int j = 0; j < NR; j++) {
-        if (r0 + j >= nrhs) break;
-        Spinor<double> v;
-        load_sp(in.p[r0 + j], Vh, 1 - par, nf, v);
-        link_spinor_acc<false>(uf, v, acc[j]);
-      }
-    }
-    {
-      const Lk ub = u.load(1 - par, mu, nb);
+    for (int d = 0; d < 2; d++) {
+      const double2* ul = d ? u.p + ((size_t)(1 - par) * 4 + mu) * 9 * Vh + nb : u.p + ((size_t)par * 4 + mu) * 9 * Vh + cb;
+      Cd w[9];
 #pragma unroll
-      for (int j = 0; j < NR; j++) {
-        if (r0 + j >= nrhs) break;
-        Spinor<double> v;
-        load_sp(in.p[r0 + j], Vh, 1 - par, nb, v);
-        link_spinor_acc<true>(ub, v, acc[j]);
+      for (int k = 0; k < 9; k++) {
+        const double2 e = __ldg(ul + (size_t)k * Vh);
+        w[k] = {e.x, e.y};
       }
+#pragma unroll
+      for (int j = 0; j < NR; j++)
+#pragma unroll
+        for (int k = 0; k < NSP; k++) {
+          Cd v[3];
+#pragma unroll
+          for (int a = 0; a < 3; a++) {
+            const double2 e = __ldg(f[j] + ((size_t)(1 - par) * 12 + k * 3 + a) * Vh + (d ? nb : nf));
+            v[a] = {e.x, e.y};
+          }
+          if (d) link_vec_acc<true>(w, v, acc[j][k]);
+          else link_vec_acc<false>(w, v, acc[j][k]);
+        }
     }
   }
 #pragma unroll
   for (int j = 0; j < NR; j++) {
     if (r0 + j >= nrhs) break;
-    Spinor<double> v;
-    load_sp(in.p[r0 + j], Vh, par, cb, v);
-    double2* o = const_cast<double2*>(out.p[r0 + j]) + (size_t)par * 12 * Vh + cb;
+    double2* o = const_cast<double2*>(out.p[r0 + j]) + ((size_t)par * 12 + s0 * 3) * Vh + cb;
+    const double2* own = f[j] + (size_t)par * 12 * Vh + cb;
 #pragma unroll
-    for (int k = 0; k < 12; k++) {
-      const Cd t = fma_s(alpha, acc[j].c[k / 3][k % 3], v.c[k / 3][k % 3]);
+    for (int k = 0; k < 3 * NSP; k++) {
+      const double2 e = __ldg(own + (size_t)k * Vh);
+      const Cd t = fma_s(alpha, acc[j][k / 3][k % 3], Cd{e.x, e.y});
       o[(size_t)k * Vh] = make_double2(norm * t.re, norm * t.im);
     }
   }

@@ -199,3 +199,17 @@ def test_propagator_argument_checks(qkx, lat48):
     with pytest.raises(qkx.QkxError) as e:
         lat48.propagator((0, 0, 0, 0), -1, 4.0)
     assert e.value.code == qkx.ERR_INVALID
+
+
+@pytest.mark.parametrize("L,n", [((2, 2, 2, 2), 1), ((6, 4, 2, 4), 2), ((6, 4, 2, 4), 3), ((10, 2, 6, 4), 4),
+                                 ((10, 2, 6, 4), 5), ((4, 4, 4, 8), 7)])
+def test_gaussian_field_groups_and_partial_blocks(qkx, oracle, L, n):
+    """1 to 7 fields: every grouping of fields a thread takes (with spare slots), and V/2 = 8 to 256, i.e.
+    partial blocks of 32 sites.  FP64 stencil, two steps: 1e-13 relative as in the tests above."""
+    U = oracle.gauge_random(L, 0.3, 61)
+    psis = [oracle.spinor_gaussian(L, 70 + i) for i in range(n)]
+    with qkx.Lattice(qkx.LatticeInfo(L=L)) as lat:
+        lat.load_smearing_gauge(U)
+        outs = lat.Gaussian_smearing(psis, nsmear=2, alpha=1.5)
+    for p, o in zip(psis, outs):
+        assert rel(o, oracle.gaussian_smear(L, U, p, 2, 1.5)) < 1e-13
