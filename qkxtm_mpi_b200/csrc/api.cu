@@ -212,7 +212,9 @@ static bool launch_hop64_tiled(qkx_ctx* c, HopArgs<SpinorF64, GaugeF64x18>& A, c
 // one FP64 18-real hop launch over A.nrhs right-hand sides (Rz: operands of EPI_XPAY_G5_RES)
 template <int B, bool DAG, int EPI>
 static int launch_hop64(qkx_ctx* c, HopArgs<SpinorF64, GaugeF64x18>& A, const HopRes& Rz = HopRes{}) {
-  if (launch_hop64_tiled<B, DAG, EPI>(c, A, Rz)) return QKX_OK;
+  if constexpr (EPI != EPI_XPAY_CGR) {
+    if (launch_hop64_tiled<B, DAG, EPI>(c, A, Rz)) return QKX_OK;
+  }
   A.nblk = s2_blocks_per_rhs(c->Vh, A.out_parity);
   // Two right-hand sides a thread share the link loads (2.60 -> 2.36 ms for 12 at 32^3x64), as long as
   // the halved grid still fills the SMs at its 6 blocks each; below that (8^3x16 with 12: 128 site
@@ -244,10 +246,16 @@ int device_status(qkx_ctx* c) {
   return QKX_ERR_CUDA;
 }
 
+// *nblk: the number of norm partials
 template <int B, bool DAG, int EPI>
 static int hop64_t(qkx_ctx* c, SpinorF64 in, SpinorF64 out, SpinorF64 x, bool x_distinct, int out_parity,
-                   double a, double cc, double s, double* norm_part) {
+                   double a, double cc, double s, double* norm_part, int* nblk = nullptr,
+                   const int* active = nullptr) {
   HopArgs<SpinorF64, GaugeF64x18> A;
+  if constexpr (EPI == EPI_XPAY_CGR) {
+    A.racc64 = out;  // the CG residual takes the place of the output
+    A.alpha = c->sc->alpha;
+  }
   A.out = out;
   A.in = in;
   A.x = x;
@@ -261,12 +269,14 @@ static int hop64_t(qkx_ctx* c, SpinorF64 in, SpinorF64 out, SpinorF64 x, bool x_
   A.nrhs = 1;
   A.cvec = nullptr;
   A.svec = nullptr;
-  A.active = nullptr;
+  A.active = active;
   const int n = out_parity < 0 ? 2 * c->Vh : c->Vh;
   QKX_TRY(prof_begin(c));
   QKX_TRY((launch_hop64<B, DAG, EPI>(c, A)));
   QKX_CUDA(cudaGetLastError());
+  if (nblk) *nblk = A.nblk;
   bool extra = (EPI == EPI_XPAY || EPI == EPI_XPAY_G5 || EPI == EPI_XPAY_TWINV) && x_distinct;
+  if (EPI == EPI_XPAY_CGR) extra = true;  // r is read and written
   return prof_end(c, hop_bytes(n, 192.0, 144.0, out_parity < 0, extra));
 }
 
@@ -685,6 +695,8 @@ void qkx_destroy(qkx_ctx* c) {
   if (c->hscal) cudaFreeHost(c->hscal);
   for (auto ev : c->ev_a) cudaEventDestroy(ev);
   for (auto ev : c->ev_b) cudaEventDestroy(ev);
+  for (auto ev : c->cg_ev)
+    if (ev) cudaEventDestroy(ev);
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
   if (c->st) cudaStreamDestroy(c->st);
@@ -851,30 +863,54 @@ int qkx_X_eq_aX_p_Y(qkx_ctx* c, double* x, double a, const double* y) {
 }
 
 // ---------------------------------------------------------------- CG (lib/solvers.cpp:16-81)
-// One run of the reference's CG recurrence on device fields, continuing from
-// the state in (r, p, sc->r2[0]) until r2 <= stop or *k reaches maxIter.
-static int cg_fp64_loop(qkx_ctx* c, double2* x, double2* r, double2* p, double2* Ap, double2* tmp, double stop,
-                        int maxIter, int* k, double* r2_host) {
+// One iteration of the reference's CG, queued: M p with |M p|^2 = <p, M^+M p> in its epilogue, alpha; then
+// M^+ M p, which goes straight into r -= alpha M^+M p and |r|^2 (it is never stored); beta and the
+// stopping rule; x += alpha p and p = r + beta p in one pass.  Against separate kernels for the
+// products, the three updates and the two dot products this moves 6 instead of 13 fields beside the
+// hops and leaves no gap for the host (16^3x32: 120 -> 83 us an iteration).
+static int cg_fp64_iteration(qkx_ctx* c, double2* x, double2* r, double2* p, double2* tmp, double* r2_slot) {
   const size_t n = 12 * c->V;
-  const int g = blas_grid(n);
+  const int Vh = c->Vh;
+  const double tw = 2.0 * c->p.kappa * c->p.mu * c->p.twistSign;
+  int nb = 0;
+  QKX_TRY((hop64_t<0, false, EPI_XPAY>(c, F64(p, Vh), F64(tmp, Vh), F64(p, Vh), false, -1, -c->p.kappa, tw, 1.0,
+                                       c->part, &nb, c->sc->active)));
+  k_cg_finalize<<<1, 1024, 0, c->st>>>(c->part, nb, FIN_PAP, c->sc, nullptr);
+  counted(c);
+  QKX_TRY((hop64_t<0, true, EPI_XPAY_CGR>(c, F64(tmp, Vh), F64(r, Vh), F64(tmp, Vh), false, -1, -c->p.kappa, -tw, 1.0,
+                                          c->part, &nb, c->sc->restart)));
+  k_cg_finalize<<<1, 1024, 0, c->st>>>(c->part, nb, FIN_R2, c->sc, r2_slot);
+  counted(c);
+  k_cg_update<<<blas_grid(n), BLAS_NT, 0, c->st>>>(c->sc, r, x, p, n);
+  counted(c);
+  QKX_CUDA(cudaGetLastError());
+  return QKX_OK;
+}
+
+// One run of the reference's CG recurrence on device fields, continuing from
+// the state in (r, p, sc->r2[0]) until r2 <= stop or *k reaches maxIter.  The host stays
+// CG_AHEAD iterations ahead of the r2 it reads, so the GPU does not wait for it.
+static int cg_fp64_loop(qkx_ctx* c, double2* x, double2* r, double2* p, double2* tmp, double stop, int maxIter, int* k,
+                        double* r2_host) {
   double r2 = *r2_host;
-  while (r2 > stop && *k < maxIter) {
-    QKX_TRY(apply_tm(c, p, tmp, false));                     // Ap.tmDagtm(p, tmp, ...)
-    QKX_TRY(apply_tm(c, tmp, Ap, true));
-    QKX_TRY(redot(c, p, Ap, n, FIN_PAP, nullptr, 0));         // pAp, alpha = r2 / pAp
-    k_axpy<<<g, BLAS_NT, 0, c->st>>>(c->sc->alpha, 1.0, p, x, n);
-    counted(c);    // x = x + alpha p
-    k_axpy<<<g, BLAS_NT, 0, c->st>>>(c->sc->alpha, -1.0, Ap, r, n);
-    counted(c);  // r = r - alpha Ap
-    QKX_CUDA(cudaGetLastError());
-    QKX_TRY(redot(c, r, r, n, FIN_R2, nullptr, 0));           // r2, beta = r2 / r2_old
-    k_xpay<<<g, BLAS_NT, 0, c->st>>>(r, c->sc->beta, p, n);
-    counted(c);          // p = r + beta p
-    QKX_CUDA(cudaGetLastError());
+  if (!(r2 > stop) || *k >= maxIter) return QKX_OK;
+  for (auto& ev : c->cg_ev)
+    if (!ev) QKX_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  double* slot = c->hscal + 8;  // page-locked, written by the device
+  k_cg_begin<<<1, 1, 0, c->st>>>(c->sc, stop);
+  counted(c);
+  long long queued = 0, read = 0;
+  const long long most = (long long)maxIter - *k;
+  while (r2 > stop && read < most) {
+    while (queued < most && queued < read + qkx_ctx::CG_AHEAD) {
+      QKX_TRY(cg_fp64_iteration(c, x, r, p, tmp, slot + queued % qkx_ctx::CG_AHEAD));
+      QKX_CUDA(cudaEventRecord(c->cg_ev[queued % qkx_ctx::CG_AHEAD], c->st));
+      queued++;
+    }
+    QKX_CUDA(cudaEventSynchronize(c->cg_ev[read % qkx_ctx::CG_AHEAD]));
+    r2 = *(volatile double*)(slot + read % qkx_ctx::CG_AHEAD);
+    read++;
     (*k)++;
-    QKX_CUDA(cudaMemcpyAsync(c->hscal, c->sc->r2, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    QKX_CUDA(cudaStreamSynchronize(c->st));
-    r2 = c->hscal[0];
     if (!(r2 == r2) || isinf(r2)) {
       *r2_host = r2;
       set_error("CG: r2 became %g at iteration %d", r2, *k);
@@ -885,17 +921,15 @@ static int cg_fp64_loop(qkx_ctx* c, double2* x, double2* r, double2* p, double2*
   return QKX_OK;
 }
 
+// r = p = in, r2 = |in|^2 (also the reference's source norm)
 static int cg_fp64_start(qkx_ctx* c, const double2* in, double2* r, double2* p, double* r2, double* src) {
   const size_t n = 12 * c->V;
   QKX_CUDA(cudaMemcpyAsync(r, in, sizeof(double2) * n, cudaMemcpyDeviceToDevice, c->st));
   QKX_CUDA(cudaMemcpyAsync(p, in, sizeof(double2) * n, cudaMemcpyDeviceToDevice, c->st));
   QKX_TRY(redot(c, r, r, n, FIN_R2_INIT, nullptr, 0));
-  QKX_TRY(redot(c, in, in, n, FIN_STORE, c->dscal, 0));
   QKX_CUDA(cudaMemcpyAsync(c->hscal, c->sc->r2, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  QKX_CUDA(cudaMemcpyAsync(c->hscal + 1, c->dscal, sizeof(double), cudaMemcpyDeviceToHost, c->st));
   QKX_CUDA(cudaStreamSynchronize(c->st));
-  *r2 = c->hscal[0];
-  *src = c->hscal[1];
+  *r2 = *src = c->hscal[0];
   return QKX_OK;
 }
 
@@ -907,17 +941,17 @@ int qkx_cg_dev(qkx_ctx* c, const double* in_dev, double* x_dev, qkx_solve_info* 
   }
   QKX_CUDA(cudaSetDevice(c->device));
   QKX_TRY(ensure_work(c));
-  double2 *r = c->w[2], *p = c->w[3], *Ap = c->w[4], *tmp = c->w[5];
+  double2 *r = c->w[2], *p = c->w[3], *tmp = c->w[5];
   const double2* in = (const double2*)in_dev;
   double2* x = (double2*)x_dev;
-  for (double2* f : {r, p, Ap, tmp})
+  for (double2* f : {r, p, c->w[4], tmp})
     if ((const double2*)in == f || x == f) return invalid("CG fields alias the context's work fields");
   QKX_CUDA(cudaEventRecord(c->t0, c->st));
   double r2, src;
   QKX_TRY(cg_fp64_start(c, in, r, p, &r2, &src));
   const double stop = src * c->p.tol * c->p.tol;
   int k = 0;
-  int rc = cg_fp64_loop(c, x, r, p, Ap, tmp, stop, c->p.maxIter, &k, &r2);
+  int rc = cg_fp64_loop(c, x, r, p, tmp, stop, c->p.maxIter, &k, &r2);
   QKX_CUDA(cudaEventRecord(c->t1, c->st));
   QKX_CUDA(cudaEventSynchronize(c->t1));
   QKX_TRY(device_status(c));
@@ -994,7 +1028,7 @@ static int invert_cg_fp64(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, con
     double rel = 0;
     int rc = QKX_OK;
     for (;;) {
-      rc = cg_fp64_loop(c, x[i], r, p, Ap, tmp, stop, sp->maxIter, &k, &r2);
+      rc = cg_fp64_loop(c, x[i], r, p, tmp, stop, sp->maxIter, &k, &r2);
       if (rc != QKX_OK) break;
       QKX_TRY(true_residual(c, b[i], x[i], &rel));
       if (rel <= sp->tol || k >= sp->maxIter || restarts >= 20) break;

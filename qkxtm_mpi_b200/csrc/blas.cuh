@@ -57,54 +57,71 @@ static __global__ void __launch_bounds__(BLAS_NT) k_redot(const double2* __restr
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// finalize modes
+// what a sum of partials is for
 enum { FIN_STORE = 0, FIN_PAP = 1, FIN_R2 = 2, FIN_R2_INIT = 3 };
 
-// Sum part[0..n) in a fixed order and act on the solver scalars of one RHS:
-//   FIN_STORE    *dst = sum
-//   FIN_PAP      pAp = sum, alpha = r2 / pAp
-//   FIN_R2       r2_old = r2, r2 = sum, beta = r2 / r2_old
-//   FIN_R2_INIT  r2 = sum
+// Sum part[0..n) in a fixed order: FIN_STORE *dst = sum; FIN_R2_INIT r2 = sum
 static __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ part, int n, double* dst,
                                                    int mode, CgScalars* sc, int rhs) {
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += 1024) acc += part[i];
   double s = block_sum<1024>(acc);
   if (threadIdx.x == 0) {
-    if (mode == FIN_STORE) {
-      *dst = s;
-    } else if (mode == FIN_PAP) {
-      sc->pAp[rhs] = s;
-      sc->alpha[rhs] = sc->r2[rhs] / s;
-    } else if (mode == FIN_R2) {
-      sc->r2_old[rhs] = sc->r2[rhs];
-      sc->r2[rhs] = s;
-      sc->beta[rhs] = s / sc->r2_old[rhs];
-    } else {
-      sc->r2[rhs] = s;
+    if (mode == FIN_STORE) *dst = s;
+    else sc->r2[rhs] = s;
+  }
+}
+
+// ---- the FP64 CG iteration (solvers.cpp:40-70) in five kernels: the two hops, the two sums and the update.
+// active[0] says whether the next iteration runs, restart[0] whether the current one does: iterations
+// the host has queued past the stopping one do nothing, so it need not wait for r2 between them.
+
+// start of the loop: the first iteration runs while r2 is above the stop
+static __global__ void k_cg_begin(CgScalars* sc, double stop) {
+  sc->stop[0] = stop;
+  sc->active[0] = sc->r2[0] > stop ? 1 : 0;
+  sc->restart[0] = 0;
+}
+
+// FIN_PAP: <p, M^+M p> = |M p|^2 from the first hop, alpha; FIN_R2: |r|^2 from the second, beta, the
+// stopping rule, and r2 to page-locked host memory
+static __global__ void __launch_bounds__(1024) k_cg_finalize(const double* __restrict__ part, int n, int mode,
+                                                      CgScalars* sc, double* r2_host) {
+  if (mode == FIN_PAP) {
+    if (!sc->active[0]) {
+      __syncthreads();
+      if (threadIdx.x == 0) sc->restart[0] = 0;
+      return;
     }
-    if (dst && mode != FIN_STORE) *dst = s;
+  } else if (!sc->restart[0]) {
+    return;
+  }
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < n; i += 1024) acc += part[i];
+  const double s = block_sum<1024>(acc);
+  if (threadIdx.x != 0) return;
+  if (mode == FIN_PAP) {
+    sc->restart[0] = 1;
+    sc->pAp[0] = s;
+    sc->alpha[0] = sc->r2[0] / s;
+  } else {
+    sc->r2_old[0] = sc->r2[0];
+    sc->r2[0] = s;
+    sc->beta[0] = s / sc->r2_old[0];
+    sc->active[0] = s > sc->stop[0] ? 1 : 0;
+    *r2_host = s;
   }
 }
 
-// y = y + a x with a = sign * (*a_dev)       (X_eq_X_p_aY, lib/blas_qkxTM.cpp:31)
-static __global__ void __launch_bounds__(BLAS_NT) k_axpy(const double* __restrict__ a_dev, double sign,
-                                                  const double2* __restrict__ x, double2* __restrict__ y,
-                                                  size_t n) {
-  const double a = sign * *a_dev;
+// x = x + alpha p, p = r + beta p in one pass (X_eq_X_p_aY and X_eq_aX_p_Y, lib/blas_qkxTM.cpp:31, 45)
+static __global__ void __launch_bounds__(BLAS_NT) k_cg_update(const CgScalars* sc, const double2* __restrict__ r,
+                                                       double2* __restrict__ x, double2* __restrict__ p, size_t n) {
+  if (!sc->restart[0]) return;
+  const double a = sc->alpha[0], b = sc->beta[0];
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
-    double2 xv = x[i], yv = y[i];
-    y[i] = make_double2(yv.x + a * xv.x, yv.y + a * xv.y);
-  }
-}
-
-// y = a y + x with a = *a_dev                (X_eq_aX_p_Y, lib/blas_qkxTM.cpp:45)
-static __global__ void __launch_bounds__(BLAS_NT) k_xpay(const double2* __restrict__ x, const double* __restrict__ a_dev,
-                                                  double2* __restrict__ y, size_t n) {
-  const double a = *a_dev;
-  for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
-    double2 xv = x[i], yv = y[i];
-    y[i] = make_double2(a * yv.x + xv.x, a * yv.y + xv.y);
+    const double2 pv = p[i], xv = x[i], rv = r[i];
+    x[i] = make_double2(xv.x + a * pv.x, xv.y + a * pv.y);
+    p[i] = make_double2(b * pv.x + rv.x, b * pv.y + rv.y);
   }
 }
 

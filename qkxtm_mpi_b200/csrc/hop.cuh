@@ -33,6 +33,8 @@ enum Epilogue {
   EPI_XPAY_G5_CGR = 7, // o = g5 (a D psi + x + i c g5 x) is not stored: the CG residual of the batch
                        // takes it, r -= alpha o, and |r|^2 goes to the norm partials (multi-RHS
                        // kernels of the mixed solver only; r is racc32, or racc64 for FP64 sloppy)
+  EPI_XPAY_CGR = 9,        // as EPI_XPAY, but o is not stored: the CG residual takes it, r -= alpha o (racc64), and
+                           // |r|^2 goes to the norm partials (hop_s2_kernel only)
   EPI_XPAY_TWINV_RES = 8,  // as EPI_XPAY_TWINV, and |v - (out + i c g5 out)|^2 to the norm partials: with
                            // x = b_o, a = kappa the odd half of ||b - M x||^2 (the same)
 };
@@ -60,7 +62,7 @@ struct HopArgs {
   const double* cvec;  // optional per-RHS factor on c (twisted mass per RHS)
   const double* svec;  // optional per-RHS factor on s
   const int* active;   // optional per-RHS mask; inactive blocks do nothing
-  // EPI_XPAY_G5_CGR only: per-RHS CG step length and the residual batch it updates
+  // EPI_XPAY_G5_CGR and EPI_XPAY_CGR: per-RHS CG step length and the residual batch it updates
   const double* alpha = nullptr;
   SpinorF32 racc32{nullptr, nullptr, 0};
   SpinorF64 racc64{nullptr, nullptr, 0};

@@ -189,6 +189,16 @@ __device__ __forceinline__ double s2_epilogue(const HopArgs<SpinorF64, GaugeF64x
         rb[2 * (size_t)(k0 >> 1) * Vh + (k0 & 1)] = make_float2(float(z0.re), float(z0.im));
         rb[2 * (size_t)(k1 >> 1) * Vh + (k1 & 1)] = make_float2(float(z1.re), float(z1.im));
       }
+    } else if constexpr (EPI == EPI_XPAY_CGR) {
+      const SpinorF64 rr = A.racc64.shift(rhs);
+      double2* rb = (par ? rr.p1 : rr.p0) + cb;
+      const double al = A.alpha[rhs];
+      double2 z0 = rb[w0], z1 = rb[w1];
+      z0 = make_double2(z0.x - al * lo.re, z0.y - al * lo.im);
+      z1 = make_double2(z1.x - al * hi.re, z1.y - al * hi.im);
+      rb[w0] = z0;
+      rb[w1] = z1;
+      nrm += z0.x * z0.x + z0.y * z0.y + z1.x * z1.x + z1.y * z1.y;
     } else {
       const SpinorF64 os = A.out.shift(rhs);
       double2* ob = (par ? os.p1 : os.p0) + cb;

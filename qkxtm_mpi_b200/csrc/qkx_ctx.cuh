@@ -74,6 +74,8 @@ struct qkx_ctx {
   int smem_optin = 0;              // shared memory a block may opt in to on this device
   int c3t = 0;                     // the TMA-tiled FP64 hop where the lattice allows it (opt-in)
   cudaEvent_t t0 = nullptr, t1 = nullptr;
+  static constexpr int CG_AHEAD = 2;  // FP64 CG iterations queued before the host reads r2 of the oldest
+  cudaEvent_t cg_ev[CG_AHEAD] = {};   // one per queued iteration
   // profiling of the hopping kernels
   int prof = 0;
   std::vector<cudaEvent_t> ev_a, ev_b;
