@@ -212,6 +212,10 @@ static bool launch_hop64_tiled(qkx_ctx* c, HopArgs<SpinorF64, GaugeF64x18>& A, c
 // one FP64 18-real hop launch over A.nrhs right-hand sides (Rz: operands of EPI_XPAY_G5_RES)
 template <int B, bool DAG, int EPI>
 static int launch_hop64(qkx_ctx* c, HopArgs<SpinorF64, GaugeF64x18>& A, const HopRes& Rz = HopRes{}) {
+  if (A.zero && c->c3t) {  // the tiled kernel does not zero on the way
+    QKX_CUDA(cudaMemsetAsync(A.zero, 0, sizeof(double2) * 12 * c->Vh, c->st));
+    A.zero = nullptr;
+  }
   if constexpr (EPI != EPI_XPAY_CGR) {
     if (launch_hop64_tiled<B, DAG, EPI>(c, A, Rz)) return QKX_OK;
   }
@@ -222,12 +226,12 @@ static int launch_hop64(qkx_ctx* c, HopArgs<SpinorF64, GaugeF64x18>& A, const Ho
   if constexpr (B == 0 && !DAG) {
     const int ngrp = (A.nrhs + 1) / 2;
     if (A.nrhs > 1 && A.nblk * ngrp >= 148 * 6) {
-      hop_s2_kernel<2, B, DAG, EPI><<<A.nblk * ngrp, 2 * S2_NS, 0, c->st>>>(A, Rz);
+      QKX_CUDA(launch_pdl(c, hop_s2_kernel<2, B, DAG, EPI>, A.nblk * ngrp, 2 * S2_NS, A, Rz));
       counted(c);
       return QKX_OK;
     }
   }
-  hop_s2_kernel<1, B, DAG, EPI><<<A.nblk * A.nrhs, 2 * S2_NS, 0, c->st>>>(A, Rz);
+  QKX_CUDA(launch_pdl(c, hop_s2_kernel<1, B, DAG, EPI>, A.nblk * A.nrhs, 2 * S2_NS, A, Rz));
   counted(c);
   return QKX_OK;
 }
@@ -250,7 +254,7 @@ int device_status(qkx_ctx* c) {
 template <int B, bool DAG, int EPI>
 static int hop64_t(qkx_ctx* c, SpinorF64 in, SpinorF64 out, SpinorF64 x, bool x_distinct, int out_parity,
                    double a, double cc, double s, double* norm_part, int* nblk = nullptr,
-                   const int* active = nullptr) {
+                   const int* active = nullptr, double2* zero = nullptr) {
   HopArgs<SpinorF64, GaugeF64x18> A;
   if constexpr (EPI == EPI_XPAY_CGR) {
     A.racc64 = out;  // the CG residual takes the place of the output
@@ -270,6 +274,7 @@ static int hop64_t(qkx_ctx* c, SpinorF64 in, SpinorF64 out, SpinorF64 x, bool x_
   A.cvec = nullptr;
   A.svec = nullptr;
   A.active = active;
+  A.zero = zero;
   const int n = out_parity < 0 ? 2 * c->Vh : c->Vh;
   QKX_TRY(prof_begin(c));
   QKX_TRY((launch_hop64<B, DAG, EPI>(c, A)));
@@ -359,10 +364,10 @@ int hop64_batch(qkx_ctx* c, int epi, int nrhs, SpinorF64 in, SpinorF64 out, Spin
 
 // runtime -> compile-time dispatch, on accessors (single-parity fields allowed)
 int hop64a(qkx_ctx* c, int basis, bool dag, int epi, SpinorF64 in, SpinorF64 out, SpinorF64 x, bool x_distinct,
-           int out_parity, double a, double cc, double s, double* norm_part) {
+           int out_parity, double a, double cc, double s, double* norm_part, double2* zero) {
 #define QKX_HOP_CASE(B_, D_, E_) \
   if (basis == B_ && dag == D_ && epi == E_)   \
-    return hop64_t<B_, D_, E_>(c, in, out, x, x_distinct, out_parity, a, cc, s, norm_part);
+    return hop64_t<B_, D_, E_>(c, in, out, x, x_distinct, out_parity, a, cc, s, norm_part, nullptr, nullptr, zero);
 #define QKX_HOP_EPIS(B_, D_) \
   QKX_HOP_CASE(B_, D_, EPI_PLAIN) QKX_HOP_CASE(B_, D_, EPI_XPAY) QKX_HOP_CASE(B_, D_, EPI_XPAY_G5) \
   QKX_HOP_CASE(B_, D_, EPI_TWIST_INV) QKX_HOP_CASE(B_, D_, EPI_XPAY_TWINV)
@@ -377,9 +382,9 @@ int hop64a(qkx_ctx* c, int basis, bool dag, int epi, SpinorF64 in, SpinorF64 out
 
 // the same on full (both-parity) fields
 static int hop64(qkx_ctx* c, int basis, bool dag, int epi, const double2* in, double2* out, const double2* x,
-                 int out_parity, double a, double cc, double s, double* norm_part = nullptr) {
+                 int out_parity, double a, double cc, double s, double2* zero = nullptr) {
   return hop64a(c, basis, dag, epi, F64(in, c->Vh), F64(out, c->Vh), F64(x ? x : in, c->Vh), x && x != in,
-                out_parity, a, cc, s, norm_part);
+                out_parity, a, cc, s, nullptr, zero);
 }
 
 int site_op_acc(qkx_ctx* c, int basis, int op, SpinorF64 in, SpinorF64 out, int par_first, int npar, double cc,
@@ -404,10 +409,8 @@ static int site_op(qkx_ctx* c, int basis, int op, const double2* in, double2* ou
   return site_op_acc(c, basis, op, F64(in, c->Vh), F64(out, c->Vh), 0, 2, cc, s);
 }
 
-static int zero_parity(qkx_ctx* c, double2* f, int parity) {
-  QKX_CUDA(cudaMemsetAsync(f + (size_t)parity * 12 * c->Vh, 0, sizeof(double2) * 12 * c->Vh, c->st));
-  return QKX_OK;
-}
+// the half of a full field with the given parity
+static double2* half_of(qkx_ctx* c, double2* f, int parity) { return f + (size_t)parity * 12 * c->Vh; }
 
 int apply_tm_mu(qkx_ctx* c, const double2* in, double2* out, bool dagger, double mu) {
   const double tw = 2.0 * c->p.kappa * mu * c->p.twistSign;
@@ -421,14 +424,15 @@ int apply_tm(qkx_ctx* c, const double2* in, double2* out, bool dagger) {
 // M_xx psi for output parity `par` (0 = EE, 1 = OO) with twist sign `sgn`:
 //   t = A^-1 D_{1-par <- par} psi ;  out_par = A psi - kappa^2 D_{par <- 1-par} t
 // (Vector::tm_xx, lib/lattice_util.cpp:2001-2022).  With g5out the result is
-// multiplied by gamma5, which is how tm_xxDagTm_xx chains two of them.
+// multiplied by gamma5, which is how tm_xxDagTm_xx chains two of them.  zero: the other parity of the
+// operator's result, set to zero by the last hop.
 static int tm_xx(qkx_ctx* c, int basis, int par, double sgn, const double2* in, double2* out, double2* tmp,
-                 bool g5out) {
+                 bool g5out, double2* zero = nullptr) {
   const double k = c->p.kappa, mu = c->p.mu;
   const double cc = 2.0 * k * mu * sgn;
   const double inv = 1.0 / (1.0 + (2.0 * k * mu) * (2.0 * k * mu));
   QKX_TRY(hop64(c, basis, false, EPI_TWIST_INV, in, tmp, nullptr, 1 - par, 0.0, cc, inv));
-  return hop64(c, basis, false, g5out ? EPI_XPAY_G5 : EPI_XPAY, tmp, out, in, par, -k * k, cc, 1.0);
+  return hop64(c, basis, false, g5out ? EPI_XPAY_G5 : EPI_XPAY, tmp, out, in, par, -k * k, cc, 1.0, zero);
 }
 
 int run_op(qkx_ctx* c, int op, const double2* in, double2* out) {
@@ -466,8 +470,7 @@ int run_op(qkx_ctx* c, int op, const double2* in, double2* out) {
     case QKX_OP_DSLASH_XX_CHIRAL_OE: {
       int basis = (op == QKX_OP_DSLASH_XX_CHIRAL_EO || op == QKX_OP_DSLASH_XX_CHIRAL_OE) ? 1 : 0;
       int par = (op == QKX_OP_DSLASH_XX_EO || op == QKX_OP_DSLASH_XX_CHIRAL_EO) ? 0 : 1;
-      QKX_TRY(hop64(c, basis, false, EPI_PLAIN, in, out, nullptr, par, 0, 0, 1));
-      return zero_parity(c, out, 1 - par);
+      return hop64(c, basis, false, EPI_PLAIN, in, out, nullptr, par, 0, 0, 1, half_of(c, out, 1 - par));
     }
     case QKX_OP_TM_XX_EE:
     case QKX_OP_TM_XX_OO:
@@ -475,8 +478,7 @@ int run_op(qkx_ctx* c, int op, const double2* in, double2* out) {
     case QKX_OP_TM_XX_CHIRAL_OO: {
       int basis = (op == QKX_OP_TM_XX_CHIRAL_EE || op == QKX_OP_TM_XX_CHIRAL_OO) ? 1 : 0;
       int par = (op == QKX_OP_TM_XX_EE || op == QKX_OP_TM_XX_CHIRAL_EE) ? 0 : 1;
-      QKX_TRY(tm_xx(c, basis, par, s, in, out, t1, false));
-      return zero_parity(c, out, 1 - par);
+      return tm_xx(c, basis, par, s, in, out, t1, false, half_of(c, out, 1 - par));
     }
     case QKX_OP_TM_XX_DAGTM_XX_EE:
     case QKX_OP_TM_XX_DAGTM_XX_OO:
@@ -486,8 +488,7 @@ int run_op(qkx_ctx* c, int op, const double2* in, double2* out) {
       int basis = (op == QKX_OP_TM_XX_DAGTM_XX_CHIRAL_EE || op == QKX_OP_TM_XX_DAGTM_XX_CHIRAL_OO) ? 1 : 0;
       int par = (op == QKX_OP_TM_XX_DAGTM_XX_EE || op == QKX_OP_TM_XX_DAGTM_XX_CHIRAL_EE) ? 0 : 1;
       QKX_TRY(tm_xx(c, basis, par, s, in, t2, t1, true));
-      QKX_TRY(tm_xx(c, basis, par, -s, t2, out, t1, true));
-      return zero_parity(c, out, 1 - par);
+      return tm_xx(c, basis, par, -s, t2, out, t1, true, half_of(c, out, 1 - par));
     }
     case QKX_OP_GAMMA5: return site_op(c, 0, SITE_GAMMA5, in, out, 0, 1);
     case QKX_OP_GAMMA5_CHIRAL: return site_op(c, 1, SITE_GAMMA5, in, out, 0, 1);
@@ -875,13 +876,13 @@ static int cg_fp64_iteration(qkx_ctx* c, double2* x, double2* r, double2* p, dou
   int nb = 0;
   QKX_TRY((hop64_t<0, false, EPI_XPAY>(c, F64(p, Vh), F64(tmp, Vh), F64(p, Vh), false, -1, -c->p.kappa, tw, 1.0,
                                        c->part, &nb, c->sc->active)));
-  k_cg_finalize<<<1, 1024, 0, c->st>>>(c->part, nb, FIN_PAP, c->sc, nullptr);
+  QKX_CUDA(launch_pdl(c, k_cg_finalize, 1, 1024, c->part, nb, FIN_PAP, c->sc, nullptr));
   counted(c);
   QKX_TRY((hop64_t<0, true, EPI_XPAY_CGR>(c, F64(tmp, Vh), F64(r, Vh), F64(tmp, Vh), false, -1, -c->p.kappa, -tw, 1.0,
                                           c->part, &nb, c->sc->restart)));
-  k_cg_finalize<<<1, 1024, 0, c->st>>>(c->part, nb, FIN_R2, c->sc, r2_slot);
+  QKX_CUDA(launch_pdl(c, k_cg_finalize, 1, 1024, c->part, nb, FIN_R2, c->sc, r2_slot));
   counted(c);
-  k_cg_update<<<blas_grid(n), BLAS_NT, 0, c->st>>>(c->sc, r, x, p, n);
+  QKX_CUDA(launch_pdl(c, k_cg_update, blas_grid(n), BLAS_NT, c->sc, r, x, p, n));
   counted(c);
   QKX_CUDA(cudaGetLastError());
   return QKX_OK;

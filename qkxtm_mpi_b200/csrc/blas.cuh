@@ -87,6 +87,7 @@ static __global__ void k_cg_begin(CgScalars* sc, double stop) {
 // stopping rule, and r2 to page-locked host memory
 static __global__ void __launch_bounds__(1024) k_cg_finalize(const double* __restrict__ part, int n, int mode,
                                                       CgScalars* sc, double* r2_host) {
+  pdl_start();
   if (mode == FIN_PAP) {
     if (!sc->active[0]) {
       __syncthreads();
@@ -116,6 +117,7 @@ static __global__ void __launch_bounds__(1024) k_cg_finalize(const double* __res
 // x = x + alpha p, p = r + beta p in one pass (X_eq_X_p_aY and X_eq_aX_p_Y, lib/blas_qkxTM.cpp:31, 45)
 static __global__ void __launch_bounds__(BLAS_NT) k_cg_update(const CgScalars* sc, const double2* __restrict__ r,
                                                        double2* __restrict__ x, double2* __restrict__ p, size_t n) {
+  pdl_start();
   if (!sc->restart[0]) return;
   const double a = sc->alpha[0], b = sc->beta[0];
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {

@@ -62,6 +62,7 @@ struct HopArgs {
   const double* cvec;  // optional per-RHS factor on c (twisted mass per RHS)
   const double* svec;  // optional per-RHS factor on s
   const int* active;   // optional per-RHS mask; inactive blocks do nothing
+  double2* zero = nullptr;  // optional [12][Vh] half field set to zero on the way (hop_s2_kernel, one right-hand side)
   // EPI_XPAY_G5_CGR and EPI_XPAY_CGR: per-RHS CG step length and the residual batch it updates
   const double* alpha = nullptr;
   SpinorF32 racc32{nullptr, nullptr, 0};

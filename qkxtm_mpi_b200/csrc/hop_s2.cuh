@@ -215,6 +215,7 @@ __device__ __forceinline__ double s2_epilogue(const HopArgs<SpinorF64, GaugeF64x
 template <int NR, int B, bool DAG, int EPI>
 __global__ void __launch_bounds__(2 * S2_NS, NR == 1 ? 8 : 6)
     hop_s2_kernel(HopArgs<SpinorF64, GaugeF64x18> A, HopRes Rz) {
+  pdl_start();
   const int ngrp = (A.nrhs + NR - 1) / NR;
   const int r0 = (blockIdx.x % ngrp) * NR;
   const int blk = blockIdx.x / ngrp;
@@ -242,6 +243,12 @@ __global__ void __launch_bounds__(2 * S2_NS, NR == 1 ? 8 : 6)
   }
   const bool inside = cb < A.g.Vh;
   if (!inside) cb = A.g.Vh - 1;  // the spare threads of the last block repeat its last site and store nothing
+  if constexpr (NR == 1 && (EPI == EPI_PLAIN || EPI == EPI_XPAY || EPI == EPI_XPAY_G5)) {
+    if (A.zero) {  // the parity that the operator leaves out
+#pragma unroll
+      for (int k = 0; k < 6; k++) A.zero[(size_t)(s * 6 + k) * A.g.Vh + cb] = make_double2(0.0, 0.0);
+    }
+  }
   const double2* in[NR];
 #pragma unroll
   for (int j = 0; j < NR; j++) {

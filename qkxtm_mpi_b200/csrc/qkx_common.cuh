@@ -22,6 +22,15 @@
 
 namespace qkx {
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// A kernel launched with launch_pdl (qkx_ctx.cuh) may be scheduled while the one before it on the stream
+// drains.  It calls pdl_start() before anything else: the next kernel may be scheduled in turn, and
+// this one waits until the kernel before it has finished and its writes are visible.  In a kernel
+// that was launched the ordinary way both instructions do nothing.
+__device__ __forceinline__ void pdl_start() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
 // ---------------------------------------------------------------- complex
 template <typename R>
 struct Cx {
