@@ -289,10 +289,10 @@ typedef struct qkx_batch_job {
 QKX_API int qkx_invert_batch(qkx_batch_job* jobs, int njobs, const qkx_solver_params* sp);
 
 /* Autotune the inner hop of CG_EO_MIXED for this lattice, precision and batch
- * size: times every tile (right-hand sides per thread x threads per block) on
- * the device and keeps the fastest for later solves (a solve with an untuned
- * (precision, nrhs) tunes itself first, outside its timed region).  No
- * reference counterpart. */
+ * size: times every tile (right-hand sides per thread x threads per block x kind) on
+ * the device and keeps the fastest for later solves.  A solve with an untuned
+ * (precision, nrhs) takes its tile by a rule on the lattice, precision and batch
+ * size.  No reference counterpart. */
 QKX_API int qkx_tune(qkx_ctx* ctx, int precision, int nrhs, int* rhs_per_thread, int* threads_per_block,
                      double* ms_per_hop);
 
@@ -306,7 +306,10 @@ QKX_API int qkx_tune(qkx_ctx* ctx, int precision, int nrhs, int* rhs_per_thread,
  * FP16 before widening to FP32 (8) and also 18-real FP32 links (9), or also
  * the link multiply in FP16 on 18-real FP16 links (10; rounds the products to
  * FP16, so qkx_tune never picks it: only qkx_set_tile selects it), or as 8
- * on 18-real FP16 links (11: no third-row rebuild).
+ * on 18-real FP16 links (11: no third-row rebuild).  Kind 12 (FP16 and FP32, tile
+ * (1, 128, 12)) splits a site over four threads by direction, for batches that
+ * do not fill the GPU; a solve of such a batch alone on the GPU then runs its
+ * inner iterations in one kernel.
  *
  * Use this tile (one of the tuner's) for later CG_EO_MIXED solves and
  * qkx_sloppy_normal calls with this precision and batch size, instead of the

@@ -47,7 +47,7 @@ struct HopRes {
   SpinorF32 res32;
 };
 
-template <class SP, class GA>
+template <class SP, class GA, class R32 = SpinorF32>
 struct HopArgs {
   SP out;
   SP in;
@@ -65,7 +65,7 @@ struct HopArgs {
   double2* zero = nullptr;  // optional [12][Vh] half field set to zero on the way (hop_s2_kernel, one right-hand side)
   // EPI_XPAY_G5_CGR and EPI_XPAY_CGR: per-RHS CG step length and the residual batch it updates
   const double* alpha = nullptr;
-  SpinorF32 racc32{nullptr, nullptr, 0};
+  R32 racc32{nullptr, nullptr, 0};
   SpinorF64 racc64{nullptr, nullptr, 0};
 };
 

@@ -79,11 +79,11 @@ __device__ __forceinline__ void hop_dir_m(const SP (&in)[NR], const GA& gauge, c
   }
 }
 
-template <int NT, int NR, class SP, class GA, typename R, int B, bool DAG, int EPI>
-__global__ void __launch_bounds__(NT) hop_mrhs_kernel(HopArgs<SP, GA> A) {
-  const int ngrp = (A.nrhs + NR - 1) / NR;
-  const int grp = blockIdx.x % ngrp;
-  const int blk = blockIdx.x / ngrp;
+// The work of one block: site block blk, group grp of NR right-hand sides.
+template <int NT, int NR, typename R, int B, bool DAG, int EPI, class ARGS>
+__device__ __forceinline__ void hop_mrhs_block(const ARGS& A, int blk, int grp) {
+  using SP = decltype(ARGS::in);
+  using GA = decltype(ARGS::gauge);
   const int r0 = grp * NR;
   bool act[NR];
   bool any = false;
@@ -171,6 +171,12 @@ __global__ void __launch_bounds__(NT) hop_mrhs_kernel(HopArgs<SP, GA> A) {
     }
   }
   if (A.norm_part) block_partials<NR, NT>(nrm, A.norm_part, A.nblk, r0, A.nrhs, blk);
+}
+
+template <int NT, int NR, class SP, class GA, typename R, int B, bool DAG, int EPI>
+__global__ void __launch_bounds__(NT) hop_mrhs_kernel(HopArgs<SP, GA> A) {
+  const int ngrp = (A.nrhs + NR - 1) / NR;
+  hop_mrhs_block<NT, NR, R, B, DAG, EPI>(A, blockIdx.x / ngrp, blockIdx.x % ngrp);
 }
 
 // blocks per RHS group for hop_mrhs_kernel (one parity)

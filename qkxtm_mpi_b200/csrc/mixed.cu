@@ -38,6 +38,7 @@
 #include "blas.cuh"
 #include "hop.cuh"
 #include "hop_mrhs.cuh"
+#include "hop_mu4.cuh"
 #include "hop_pair.cuh"
 #include "hop_c3t.cuh"
 #include "qkx_ctx.cuh"
@@ -49,6 +50,7 @@ namespace qkx {
 struct PHalf {
   static constexpr int id = QKX_PREC_HALF;
   using SP = SpinorF16;
+  using SPC = SpinorF16T<LdCg>;
   using GA = GaugeF16x12;
   using R = float;
   using AC = SpinorF32;
@@ -59,6 +61,7 @@ struct PHalf {
 struct PSingle {
   static constexpr int id = QKX_PREC_SINGLE;
   using SP = SpinorF32;
+  using SPC = SpinorF32T<LdCg>;
   using GA = GaugeF32x12;
   using R = float;
   using AC = SpinorF32;
@@ -143,6 +146,12 @@ static SpinorF64 B64full(double2* even, double2* odd, int Vh) {
   s.rs = 12 * (size_t)Vh;
   return s;
 }
+
+// the same field read from L2 (LdCg)
+static inline SpinorF16T<LdCg> l2_reads(const SpinorF16& f) {
+  return SpinorF16T<LdCg>{f.p0, f.p1, f.n0, f.n1, f.Vh, f.rs, f.rsn};
+}
+static inline SpinorF32T<LdCg> l2_reads(const SpinorF32& f) { return SpinorF32T<LdCg>{f.p0, f.p1, f.Vh, f.rs}; }
 
 template <class SPT>
 static int bfield_alloc(BField& f, int R, int Vh) {
@@ -417,6 +426,223 @@ __global__ void __launch_bounds__(MAX_RHS) k_ctl_after_iter(const CgScalars* sc,
   }
 }
 
+// ---------------------------------------------------------------- inner loop of a small lattice in one kernel
+// On a small lattice an iteration is eight kernels of 2-5 us that mostly wait: for their launch, for
+// round trips to memory, and for the last block.  This kernel is the whole inner loop of such a
+// solve: a cooperative grid of 128-thread blocks, each with its fixed (32 sites, right-hand side)
+// items, runs iterations until k_ctl_after_iter's decision, with a grid barrier between the steps.
+// Every block sums the norm partials itself (in k_mx_finalize's order) and takes the decisions from the
+// same numbers, so no scalar travels between kernels.  The hops are hop_mu4_block's and the update is
+// k_mx_update_p's, so the bits are those of the kernel-by-kernel loop with tile kind 12.
+// Fields that blocks exchange are read from L2 (LdCg).
+// 8^3x16, one source, FP16: 33 -> 20 us an iteration (five barriers of about 1.3 us), the solve of 32
+// iterations 1.60 -> 1.23 ms; three sources 1.69 -> 1.41; 6^3x12 1.51 -> 1.16; 12x14x10x18 1.71 -> 1.46 ms.
+// With a fence, an arrival counter and a generation word instead of one growing counter, 1.39 ms.
+template <class SP, class AC, class GA>
+struct InnerArgs {
+  SP p, t, y;
+  AC xs, rs;
+  GA U;
+  Geom g;
+  double k2;
+  int nrhs, nblk;
+  double* part;
+  const double *cvec, *svec;
+  CgScalars* sc;
+  MxCtl* ctl;
+  unsigned long long* bar;  // arrivals at the grid barrier
+  int* err;       // the context's status word
+};
+
+constexpr int SMALL_ITEMS = 148 * 4;
+constexpr unsigned long long INNER_WAIT_NS = 2000000000ull;  // longest wait at a grid barrier
+
+// The blocks of a cooperative grid meet at a counter that only grows: each adds one (release) and thread 0 polls
+// (acquire) until everybody has.  Starts from the multiple of the grid size at or below the counter,
+// which fewer than gridDim.x blocks can have passed when a block begins.
+struct GridBarrier {
+  unsigned long long* count;
+  unsigned long long target;
+  int* err;
+  __device__ __forceinline__ GridBarrier(unsigned long long* c, int* e) : count(c), target(0), err(e) {
+    if (threadIdx.x == 0) {
+      const unsigned long long v = peek();
+      target = v - v % gridDim.x;
+    }
+  }
+  __device__ __forceinline__ unsigned long long peek() const {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
+    return v;
+  }
+  // false (and a code in *err) when a block does not arrive in time
+  __device__ __forceinline__ bool meet() {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      target += gridDim.x;
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(count), "l"(1ull) : "memory");
+      int good = 1;
+      unsigned polls = 0;
+      unsigned long long t0 = 0;
+      while (peek() < target) {
+        if ((++polls & 255u) == 0) {
+          const unsigned long long t = mx_clock_ns();
+          if (t0 == 0) t0 = t;
+          if (t - t0 > INNER_WAIT_NS) {
+            atomicCAS(err, 0, 2);
+            good = 0;
+            break;
+          }
+        }
+      }
+      ok = good;
+    }
+    __syncthreads();
+    return ok != 0;
+  }
+};
+
+// sum of part[0..n), by one warp, in the order of k_mx_finalize's block of 256 threads: a[v] is its warp v
+__device__ __forceinline__ double sum_partials_warp(const double* part, int n, int lane) {
+  double a[8] = {};
+  for (int i0 = 0; i0 < n; i0 += 256) {  // eight loads in flight
+    double b[8];
+#pragma unroll
+    for (int v = 0; v < 8; v++) b[v] = i0 + v * 32 + lane < n ? __ldcg(part + i0 + v * 32 + lane) : 0.0;
+#pragma unroll
+    for (int v = 0; v < 8; v++) a[v] += b[v];
+  }
+#pragma unroll
+  for (int v = 0; v < 8; v++)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a[v] += __shfl_xor_sync(0xffffffffu, a[v], o);
+  return ((a[0] + a[4]) + (a[2] + a[6])) + ((a[1] + a[5]) + (a[3] + a[7]));
+}
+
+template <class SP, class AC, class GA, typename R>
+__global__ void __launch_bounds__(128) k_inner_small(InnerArgs<SP, AC, GA> A) {
+  __shared__ double r2[MAX_RHS], alpha[MAX_RHS], beta[MAX_RHS];
+  __shared__ int active[MAX_RHS], any, ru, bad;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, items = A.nblk * A.nrhs;
+  const bool first = blockIdx.x == 0 && tid == 0;  // writes the scalars back
+  for (int i = tid; i < A.nrhs; i += 128) {
+    r2[i] = A.sc->r2[i];
+    active[i] = A.sc->active[i];
+    alpha[i] = beta[i] = 0.0;
+  }
+  GridBarrier grid(A.bar, A.err);
+  int iter = A.ctl->iter, since = A.ctl->since;
+  const int maxIter = A.ctl->maxIter;
+  __syncthreads();
+  HopArgs<SP, GA, AC> H;
+  H.gauge = A.U;
+  H.g = A.g;
+  H.nrhs = A.nrhs;
+  H.nblk = A.nblk;
+  H.cvec = A.cvec;
+  H.active = active;
+  H.alpha = alpha;
+  H.s = 1.0;
+  H.racc32 = A.rs;
+  for (;;) {
+    // t_o = A^-1(c) D p
+    H.in = A.p, H.x = A.p, H.out = A.t, H.out_parity = 1, H.a = 0.0, H.c = 1.0, H.svec = A.svec, H.norm_part = nullptr;
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+      hop_mu4_block<EPI_TWIST_INV>(H, it / A.nrhs, it % A.nrhs);
+      __syncthreads();
+    }
+    if (!grid.meet()) break;
+    // y_e = g5 (A(c) p - k^2 D t), |y|^2
+    H.in = A.t, H.out = A.y, H.out_parity = 0, H.a = -A.k2, H.svec = nullptr, H.norm_part = A.part;
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+      hop_mu4_block<EPI_XPAY_G5>(H, it / A.nrhs, it % A.nrhs);
+      __syncthreads();
+    }
+    if (!grid.meet()) break;
+    if (tid == 0) any = ru = bad = 0;
+    for (int r = warp; r < A.nrhs; r += 4) {  // a warp a right-hand side
+      if (!active[r]) continue;
+      const double s = sum_partials_warp(A.part + (size_t)r * A.nblk, A.nblk, lane);
+      if (lane == 0) {
+        alpha[r] = r2[r] / s;
+        if (blockIdx.x == 0) {
+          A.sc->pAp[r] = s;
+          A.sc->alpha[r] = r2[r] / s;
+        }
+      }
+    }
+    // t_o = A^-1(-c) D y
+    H.in = A.y, H.x = A.y, H.out = A.t, H.out_parity = 1, H.a = 0.0, H.c = -1.0, H.svec = A.svec, H.norm_part = nullptr;
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+      hop_mu4_block<EPI_TWIST_INV>(H, it / A.nrhs, it % A.nrhs);
+      __syncthreads();
+    }
+    if (!grid.meet()) break;
+    // r -= alpha g5 (A(-c) y - k^2 D t), |r|^2
+    H.in = A.t, H.out = A.t, H.out_parity = 0, H.a = -A.k2, H.svec = nullptr, H.norm_part = A.part;
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+      hop_mu4_block<EPI_XPAY_G5_CGR>(H, it / A.nrhs, it % A.nrhs);
+      __syncthreads();
+    }
+    if (!grid.meet()) break;
+    iter++;
+    since++;
+    for (int r = warp; r < A.nrhs; r += 4) {  // with k_ctl_after_iter's tests
+      if (!active[r]) continue;
+      const double s = sum_partials_warp(A.part + (size_t)r * A.nblk, A.nblk, lane);
+      if (lane != 0) continue;
+      const double old = r2[r];
+      beta[r] = s / old;
+      r2[r] = s;
+      const bool nan = !(s == s) || isinf(s);
+      atomicOr(&any, 1);
+      if (nan) atomicOr(&bad, 1);
+      if (s < A.ctl->delta2 * A.ctl->r2ru[r] || s * A.ctl->ratio[r] <= A.ctl->target2 * A.ctl->bnorm2[r]) atomicOr(&ru, 1);
+      if (blockIdx.x == 0) {
+        A.sc->r2_old[r] = old;
+        A.sc->r2[r] = s;
+        A.sc->beta[r] = s / old;
+        A.sc->iters[r] += 1;
+        A.ctl->r2rec[r] = s;
+        if (nan) {
+          atomicMin(&A.ctl->nan_rhs, r);
+          atomicCAS(&A.ctl->nan_iter, 0, iter);
+        }
+      }
+    }
+    __syncthreads();
+    // x += alpha p, p = r + beta p; a thread a site, over the whole grid (r is complete since the last barrier)
+    const int n = A.g.Vh * A.nrhs;
+    for (int j = blockIdx.x * 128 + tid; j < n; j += gridDim.x * 128) {
+      const int r = j / A.g.Vh, cb = j - r * A.g.Vh;
+      if (!active[r]) continue;
+      const R al = R(alpha[r]), be = R(beta[r]);
+      const SP pr = A.p.shift(r);
+      const AC xr = A.xs.shift(r), rr = A.rs.shift(r);
+      Spinor<R> pv = pr.load(0, cb), rv = rr.load(0, cb), xv = xr.load(0, cb);
+#pragma unroll
+      for (int k = 0; k < 12; k++) {
+        Cx<R>& X = xv.c[k / 3][k % 3];
+        X = X + al * pv.c[k / 3][k % 3];
+        pv.c[k / 3][k % 3] = rv.c[k / 3][k % 3] + be * pv.c[k / 3][k % 3];
+      }
+      xr.store(0, cb, xv);
+      pr.store(0, cb, pv);
+    }
+    if (!(any && !ru && !bad && since < 200 && iter < maxIter)) {
+      if (first) {
+        A.ctl->iter = iter;
+        A.ctl->since = since;
+        A.ctl->t_ru0 = mx_clock_ns();
+      }
+      return;
+    }
+    if (!grid.meet()) break;
+  }
+  if (first) A.ctl->iter = maxIter;  // a barrier gave up: no further pass (the status word voids the solve)
+}
+
 // after a reliable update (|rhat|^2 in aux, |Mh^+ rhat|^2 in aux2): converged and diverged RHS
 // stop, the others restart their sloppy recursion from the new residual; the outer loop goes
 // on while any RHS is active, below maxIter, with finite residuals
@@ -470,11 +696,12 @@ __global__ void __launch_bounds__(MAX_RHS) k_ctl_final(CgScalars* sc, MxCtl* ctl
 // of their own branch): emit(part, h_outer, h_inner) launches the kernels of each part on the
 // context's stream while it is being captured (-1: top level, before anything else of the
 // branch; 0: top level before the outer loop; 4: top level after it; 1: outer body before the
-// inner loop; 2: outer body after it; 3: inner body).  The kernels each level launched come back
-// in *kt, *ko, *ki.  Both handles default to 0 at every launch, so a loop whose condition is never
+// inner loop; 2: outer body after it; 3: inner body; 5: the inner loop as one kernel, when
+// `inner_kernel`).  The kernels each level launched come back in *kt, *ko, *ki.  Both handles default to 0 at every launch, so a loop whose condition is never
 // set does not run.
 template <class Emit>
-static int build_loop_graph(qkx_ctx* c, cudaGraph_t top, long long* kt, long long* ko, long long* ki, Emit emit) {
+static int build_loop_graph(qkx_ctx* c, cudaGraph_t top, bool inner_kernel, long long* kt, long long* ko,
+                            long long* ki, Emit emit) {
   bool capturing = false;
   auto begin = [&](cudaGraph_t g) -> int {
     QKX_CUDA(cudaStreamBeginCaptureToGraph(c->st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
@@ -523,6 +750,13 @@ static int build_loop_graph(qkx_ctx* c, cudaGraph_t top, long long* kt, long lon
     QKX_TRY(add_while(h_outer, &outer_body));
     QKX_TRY(emit(4, h_outer, h_inner));
     QKX_TRY(end(kt));
+    if (inner_kernel) {
+      *ki = 0;
+      QKX_TRY(begin(outer_body));
+      QKX_TRY(emit(5, h_outer, h_inner));
+      QKX_TRY(emit(2, h_outer, h_inner));
+      return end(ko);
+    }
     QKX_CUDA(cudaGraphConditionalHandleCreate(&h_inner, outer_body, 0, cudaGraphCondAssignDefault));
     QKX_TRY(begin(outer_body));
     QKX_TRY(emit(1, h_outer, h_inner));
@@ -555,10 +789,12 @@ struct MixedState {
   double* cvec = nullptr;  // per-RHS 2 kappa mu_r twistSign
   double* svec = nullptr;  // per-RHS 1 / (1 + (2 kappa mu_r)^2)
   double* part = nullptr;  // [R][max(nblk, MX_GRID)]
+  unsigned long long* bar = nullptr;  // grid barrier of the inner loop's kernel
   MxCtl* ctl = nullptr;    // decisions of the device-driven loop
   MxCtl* ctl_h = nullptr;  // page-locked host copy
   cudaGraphExec_t dgraph = nullptr;  // the device-driven iteration loop
   int dgraph_R = 0, dgraph_nr = 0, dgraph_nt = 0, dgraph_kind = 0;
+  bool dgraph_inner = false;   // built with the inner loop as one kernel
   double dgraph_kappa = 0;
   long long dgraph_k[3] = {};  // kernels of its top level, outer pass, inner pass
   cudaGraphExec_t graph = nullptr;  // one iteration (host-driven loop)
@@ -582,6 +818,7 @@ void mixed_free(qkx_ctx* c) {
   if (m->graph) cudaGraphExecDestroy(m->graph);
   if (m->dgraph) cudaGraphExecDestroy(m->dgraph);
   cudaFree(m->ctl);
+  cudaFree(m->bar);
   if (m->ctl_h) cudaFreeHost(m->ctl_h);
   for (auto e : m->gev) cudaEventDestroy(e);
   for (auto e : m->ph)
@@ -624,6 +861,7 @@ static int mixed_alloc(qkx_ctx* c, int R, bool solver) {
     for (double2** f : {&m->bE, &m->bO, &m->x64, &m->g5bh, &m->t64, &m->z64, &m->r64})
       if (rc == QKX_OK && !*f && cudaMalloc(f, h64) != cudaSuccess) rc = QKX_ERR_NOMEM;
     if (rc == QKX_OK && !m->ctl && cudaMalloc(&m->ctl, sizeof(MxCtl)) != cudaSuccess) rc = QKX_ERR_NOMEM;
+    if (rc == QKX_OK && !m->bar && cudaMalloc(&m->bar, sizeof(unsigned long long)) != cudaSuccess) rc = QKX_ERR_NOMEM;
     if (rc == QKX_OK && !m->ctl_h && cudaMallocHost(&m->ctl_h, sizeof(MxCtl)) != cudaSuccess) rc = QKX_ERR_NOMEM;
   }
   if (rc != QKX_OK) {
@@ -653,6 +891,8 @@ static int mixed_alloc(qkx_ctx* c, int R, bool solver) {
 //      update on a 32^3x64 batch, so the tuner does not pick it; qkx_set_tile does.
 //  11  as 8 with the 18-real FP16 links (boundary sign included): nine half2
 //      conversions a link and no third-row rebuild, for 12 more bytes a link.
+//  12  hop_mu4_kernel (FP16 and FP32): a site split over four threads by direction, one
+//      right-hand side a thread, 32 sites a block.
 struct HopTile {
   int nr = 0, nt = 0, kind = 0;
 };
@@ -662,7 +902,7 @@ static const HopTile kTiles[] = {{1, 64, 0}, {1, 128, 0}, {1, 256, 0}, {2, 64, 0
                                  {2, 64, 3}, {2, 128, 3}, {2, 64, 4}, {2, 128, 4}, {2, 256, 4}, {2, 64, 5},
                                  {2, 128, 5}, {2, 64, 6}, {2, 64, 7}, {2, 128, 7}, {2, 64, 8}, {2, 128, 8},
                                  {2, 64, 9},  {2, 128, 9}, {2, 64, 10}, {2, 128, 10}, {2, 64, 11},
-                                 {2, 128, 11}};
+                                 {2, 128, 11}, {1, 128, 12}};
 
 template <int NT, int NR, int KIND, class SP, class GA, typename R, int EPI>
 static int launch_mrhs(qkx_ctx* c, int R_, const GA& gauge, const Geom& g, SP in, SP out, SP x, int out_parity,
@@ -680,7 +920,7 @@ static int launch_mrhs(qkx_ctx* c, int R_, const GA& gauge, const Geom& g, SP in
   A.s = 1.0;
   A.norm_part = norm_part;
   A.nrhs = R_;
-  A.nblk = mrhs_site_blocks<NT>(c->Vh);
+  A.nblk = mrhs_site_blocks<(KIND == 12 ? MU4_NS : NT)>(c->Vh);
   A.cvec = m->cvec;
   A.svec = with_s ? m->svec : nullptr;
   A.active = c->sc->active;
@@ -695,7 +935,10 @@ static int launch_mrhs(qkx_ctx* c, int R_, const GA& gauge, const Geom& g, SP in
   constexpr bool f16 = std::is_same<SP, SpinorF16>::value && std::is_same<GA, GaugeF16x12>::value;
   // blocks an SM must hold: 65536 registers / (128 or about 100 a thread x NT)
   constexpr int B128 = 512 / NT, B100 = 640 / NT;
-  if constexpr (KIND >= 1 && KIND <= 3) {
+  if constexpr (KIND == 12) {
+    static_assert(NR == 1 && NT == 4 * MU4_NS, "one right-hand side a thread, 32 sites a block");
+    hop_mu4_kernel<SP, GA, EPI><<<A.nblk * R_, NT, 0, c->st>>>(A);
+  } else if constexpr (KIND >= 1 && KIND <= 3) {
     static_assert(f16 && NR == 2, "pipelined tiles are FP16 pairs");
     constexpr int MINB = KIND == 1 ? 0 : (KIND == 2 ? B128 : B100);
     hop_pair_pf_kernel<NT, MINB, 0, false, EPI><<<A.nblk * ngrp, NT, 0, c->st>>>(A);
@@ -757,6 +1000,9 @@ static int hop_tile(qkx_ctx* c, HopTile t, int R_, const GA& gauge, const Geom& 
     QKX_TILE(2, 64, 10) QKX_TILE(2, 128, 10)
     QKX_TILE(2, 64, 11) QKX_TILE(2, 128, 11)
   }
+  if constexpr (!std::is_same<R, double>::value && (EPI == EPI_TWIST_INV || EPI == EPI_XPAY_G5 || EPI == EPI_XPAY_G5_CGR)) {
+    QKX_TILE(1, 128, 12)
+  }
 #undef QKX_TILE
   set_error("invalid hop tile (%d, %d, kind %d) for this precision", t.nr, t.nt, t.kind);
   return QKX_ERR_INVALID;
@@ -781,7 +1027,8 @@ struct Sloppy {
     SP p = FT::acc(m->p, 0, Vh), t = FT::acc(m->t, 1, Vh), y = FT::acc(m->y, 0, Vh), Ap = FT::acc(m->Ap, 0, Vh);
     AC xs = FA::acc(m->xs, 0, Vh), rs = FA::acc(m->rs, 0, Vh);
     const double k2 = c->p.kappa * c->p.kappa;
-    const int nblk = (Vh + tile.nt - 1) / tile.nt;
+    const int ns = tile.kind == 12 ? MU4_NS : tile.nt;  // sites a block
+    const int nblk = (Vh + ns - 1) / ns;
     const GA U = gauge(c);
     const Geom g = geom(c);
     QKX_TRY((hop_tile<SP, GA, R, EPI_TWIST_INV>(c, tile, R_, U, g, p, t, p, 1, 0.0, +1.0, true, nullptr,
@@ -802,6 +1049,54 @@ struct Sloppy {
     counted(c);
     QKX_CUDA(cudaGetLastError());
     return QKX_OK;
+  }
+
+  // the inner loop as one cooperative kernel (FP16 and FP32 sloppy, tile kind 12)
+  static int inner_small(qkx_ctx* c, int R_) {
+    if constexpr (P::id == QKX_PREC_DOUBLE) {
+      set_error("internal: no inner-loop kernel for FP64");
+      return QKX_ERR_INVALID;
+    } else {
+      using SPC = typename P::SPC;
+      using ACC = SpinorF32T<LdCg>;
+      MixedState* m = c->mixed;
+      using FT = FieldTraits<SP>;
+      using FA = FieldTraits<AC>;
+      const int Vh = c->Vh;
+      InnerArgs<SPC, ACC, GA> A;
+      A.p = l2_reads(FT::acc(m->p, 0, Vh));
+      A.t = l2_reads(FT::acc(m->t, 1, Vh));
+      A.y = l2_reads(FT::acc(m->y, 0, Vh));
+      A.xs = l2_reads(FA::acc(m->xs, 0, Vh));
+      A.rs = l2_reads(FA::acc(m->rs, 0, Vh));
+      A.U = gauge(c);
+      A.g = geom(c);
+      A.k2 = c->p.kappa * c->p.kappa;
+      A.nrhs = R_;
+      A.nblk = mrhs_site_blocks<MU4_NS>(Vh);
+      A.part = m->part;
+      A.cvec = m->cvec;
+      A.svec = m->svec;
+      A.sc = c->sc;
+      A.ctl = m->ctl;
+      A.bar = m->bar;
+      A.err = c->dstat;
+      int per_sm = 0, sms = 0;
+      QKX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_inner_small<SPC, ACC, GA, R>, 128, 0));
+      QKX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = std::min(A.nblk * R_, per_sm * sms);
+      cfg.blockDim = 128;
+      cfg.stream = c->st;
+      cudaLaunchAttribute at = {};
+      at.id = cudaLaunchAttributeCooperative;
+      at.val.cooperative = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      QKX_CUDA(cudaLaunchKernelEx(&cfg, k_inner_small<SPC, ACC, GA, R>, A));
+      counted(c);
+      return QKX_OK;
+    }
   }
 
   // algorithmic bytes of one of the four inner hops, averaged, per RHS in a batch of R_:
@@ -866,7 +1161,7 @@ static int tune_tile(qkx_ctx* c, int R_, HopTile* best, double* best_ms) {
   std::vector<std::array<double, 4>> log;
   for (const HopTile& tile : kTiles) {
     if (tile.nr > 1 && tile.nr > R_) continue;
-    if (tile.kind != 0 && P::id != QKX_PREC_HALF) continue;
+    if (tile.kind != 0 && P::id != QKX_PREC_HALF && !(tile.kind == 12 && P::id == QKX_PREC_SINGLE)) continue;
     if (tile.kind == 10) continue;  // changes the rounding of the operator, chosen explicitly only
     for (int rep = 0; rep < 4 && rc == QKX_OK; rep++) {
       if (rep == 1) rc = cudaEventRecord(e0, c->st) == cudaSuccess ? QKX_OK : QKX_ERR_CUDA;
@@ -902,17 +1197,32 @@ static int tune_tile(qkx_ctx* c, int R_, HopTile* best, double* best_ms) {
   return rc;
 }
 
+// A batch whose inner loop runs as one kernel (k_inner_small): at most four items of 32 sites an SM.  Solves of
+// 41 to 473 items gain 15-35% (at the kernel); at 640 to 648 (8^3x16 with five right-hand sides, 12^3x24 with
+// one) the two ways take the same time, and above that the tiles that fill the GPU win.
+static bool small_batch(const qkx_ctx* c, int R_) { return mrhs_site_blocks<MU4_NS>(c->Vh) * R_ <= SMALL_ITEMS; }
+
+// The tile of a solve: the one qkx_tune or qkx_set_tile recorded for this precision and batch size, else by
+// rule.  On lattices from 6^3x12 to 32^3x64 and batches of 1 to 12 these were the tuner's choice or within
+// 3% of it (12 right-hand sides at 32^3x64: FP16 0.737 ms a hop with (2, 64, 11) against 1.07 with (1, 64, 0);
+// FP32 1.165 with (1, 64, 0) against 1.208 with (2, 128, 0)), so a first solve does not time tiles.
+// alone: the solve has the GPU to itself (the branches of a batch of lattices have not, and run kernel by kernel).
 template <class P>
-static int tile_for(qkx_ctx* c, int R_, HopTile* tile) {
+static int tile_for(qkx_ctx* c, int R_, HopTile* tile, bool alone = true) {
   auto it = c->tuned.find(P::id * 1000 + R_);
+  const bool small = alone && small_batch(c, R_);
   if (it != c->tuned.end()) {
     tile->nr = it->second.nr;
     tile->nt = it->second.nt;
     tile->kind = it->second.kind;
-    return QKX_OK;
+  } else if (P::id == QKX_PREC_HALF) {
+    *tile = small ? HopTile{1, 128, 12} : (R_ == 1 ? HopTile{1, 64, 0} : HopTile{2, 64, 11});
+  } else if (P::id == QKX_PREC_SINGLE) {
+    *tile = small ? HopTile{1, 128, 12} : HopTile{1, 64, 0};
+  } else {
+    *tile = R_ == 1 ? HopTile{1, 256, 0} : HopTile{2, 128, 0};
   }
-  double ms;
-  return tune_tile<P>(c, R_, tile, &ms);
+  return QKX_OK;
 }
 
 // ---------------------------------------------------------------- batched FP64 pieces
@@ -1000,6 +1310,7 @@ struct MixedSolve {
   int maxIter = 0;
   dim3 cg2, bg2;
   bool device_loop = false;
+  bool inner_kernel = false;  // the inner loop is one kernel
   long long kcount[3] = {};  // kernels of the loop graph's top level, outer pass and inner pass
   // results of the host-driven loop (the device loop keeps them in MxCtl)
   int iter = 0, n_ru = 0, n_restart = 0, diverged = 0, nact = 0;
@@ -1010,10 +1321,12 @@ struct MixedSolve {
   MixedSolve(qkx_ctx* c_, const qkx_solver_params* sp_, int nrhs_, const double2* const* b_, double2* const* x_)
       : c(c_), sp(sp_), nrhs(nrhs_), b(b_), x(x_), active(nrhs_, 1), bnorm2(nrhs_) {}
 
-  int prepare(bool allow_device_loop) {
+  // alone: nothing else is meant to run on the GPU beside this solve (a batch of lattices is not alone,
+  // and a cooperative kernel would wait for room for its whole grid)
+  int prepare(bool allow_device_loop, bool alone) {
     QKX_TRY(mixed_alloc<P>(c, nrhs, true));
     m = c->mixed;
-    QKX_TRY(tile_for<P>(c, nrhs, &tile));
+    QKX_TRY(tile_for<P>(c, nrhs, &tile, alone));
     Vh = c->Vh;
     n12 = 12 * (size_t)Vh;
     hb = sizeof(double2) * n12;
@@ -1027,6 +1340,7 @@ struct MixedSolve {
     // the whole iteration loop on the device (one graph launch) unless the hop kernels are being
     // timed one by one (event records cannot sit inside a conditional graph body) or graphs are off
     device_loop = allow_device_loop && sp->use_graphs != 0 && c->prof == 0;
+    inner_kernel = device_loop && alone && tile.kind == 12 && small_batch(c, nrhs);
     MxCtl* hc = m->ctl_h;
     memset(hc, 0, sizeof(MxCtl));
     hc->nrhs = nrhs;
@@ -1053,6 +1367,7 @@ struct MixedSolve {
     QKX_CUDA(cudaMemcpyAsync(m->svec, hc->sv, sizeof(double) * nrhs, cudaMemcpyHostToDevice, c->st));
     QKX_CUDA(cudaMemcpyAsync(c->sc, c->sc_h, sizeof(CgScalars), cudaMemcpyHostToDevice, c->st));
     if (device_loop) QKX_CUDA(cudaMemcpyAsync(m->ctl, hc, sizeof(MxCtl), cudaMemcpyHostToDevice, c->st));
+    if (inner_kernel) QKX_CUDA(cudaMemsetAsync(m->bar, 0, sizeof(unsigned long long), c->st));
     for (int i = 0; i < nrhs; i++) {
       QKX_CUDA(cudaMemcpyAsync(m->bE + i * n12, b[i], hb, cudaMemcpyDeviceToDevice, c->st));
       QKX_CUDA(cudaMemcpyAsync(m->bO + i * n12, b[i] + n12, hb, cudaMemcpyDeviceToDevice, c->st));
@@ -1159,10 +1474,11 @@ struct MixedSolve {
   // into the top level before and after the loop (the batch's set-up and final phase).
   template <class Pre, class Post>
   int loop_graph(cudaGraph_t top, long long* kt, long long* ko, long long* ki, Pre pre, Post post) {
-    return build_loop_graph(c, top, kt, ko, ki,
+    return build_loop_graph(c, top, inner_kernel, kt, ko, ki,
                             [&](int part, cudaGraphConditionalHandle h_outer, cudaGraphConditionalHandle h_inner) -> int {
                               if (part == -1) return pre();
                               if (part == 4) return post();
+                              if (part == 5) return SL::inner_small(c, nrhs);
                               if (part == 0) {  // per-RHS state from the set-up
                                 k_ctl_start<<<1, MAX_RHS, 0, c->st>>>(c->sc, m->ctl, h_outer);
                                 counted(c);
@@ -1190,7 +1506,7 @@ struct MixedSolve {
   // the loop graph of this context (cached while the batch size, kappa and tile stay), launched
   int device_loop_launch() {
     if (m->dgraph && (m->dgraph_R != nrhs || m->dgraph_kappa != c->p.kappa || m->dgraph_nr != tile.nr ||
-                      m->dgraph_nt != tile.nt || m->dgraph_kind != tile.kind)) {
+                      m->dgraph_nt != tile.nt || m->dgraph_kind != tile.kind || m->dgraph_inner != inner_kernel)) {
       QKX_CUDA(cudaStreamSynchronize(c->st));
       cudaGraphExecDestroy(m->dgraph);
       m->dgraph = nullptr;
@@ -1216,6 +1532,7 @@ struct MixedSolve {
       m->dgraph_nr = tile.nr;
       m->dgraph_nt = tile.nt;
       m->dgraph_kind = tile.kind;
+      m->dgraph_inner = inner_kernel;
       m->dgraph_k[0] = kt;
       m->dgraph_k[1] = ko;
       m->dgraph_k[2] = ki;
@@ -1477,7 +1794,7 @@ template <class P>
 static int invert_eo_mixed_t(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double2* const* b,
                              double2* const* x, qkx_solve_info* info) {
   MixedSolve<P> s(c, sp, nrhs, b, x);
-  QKX_TRY(s.prepare(true));
+  QKX_TRY(s.prepare(true, true));
   MixedState* m = c->mixed;
   QKX_CUDA(cudaEventRecord(c->t0, c->st));
   QKX_TRY(s.setup());
@@ -1525,7 +1842,7 @@ static int batch_graph_t(std::vector<BatchGroup>& groups, qkx_batch_job* jobs, c
   std::vector<std::unique_ptr<MixedSolve<P>>> solves;
   for (BatchGroup& g : groups) {
     solves.emplace_back(new MixedSolve<P>(g.c, &g.p, (int)g.b.size(), g.b.data(), g.x.data()));
-    QKX_TRY(solves.back()->prepare(true));
+    QKX_TRY(solves.back()->prepare(true, false));
     if (!solves.back()->device_loop) {
       set_error("internal: the batch graph needs the device-driven loop");
       return QKX_ERR_INVALID;
@@ -1737,7 +2054,9 @@ static int sloppy_normal_t(qkx_ctx* c, int R_, HopTile tile, const double* const
 
 static bool known_tile(int precision, int nr, int nt, int kind) {
   for (const HopTile& t : kTiles)
-    if (t.nr == nr && t.nt == nt && t.kind == kind && (kind == 0 || precision == QKX_PREC_HALF)) return true;
+    if (t.nr == nr && t.nt == nt && t.kind == kind &&
+        (kind == 0 || precision == QKX_PREC_HALF || (kind == 12 && precision == QKX_PREC_SINGLE)))
+      return true;
   set_error("invalid argument: tile (%d, %d, kind %d) is not one of the tuner's tiles for this precision", nr, nt,
             kind);
   return false;

@@ -298,6 +298,17 @@ __device__ __forceinline__ int cb_neighbour(const Geom& g, const int x[4], int m
 }
 
 // ---------------------------------------------------------------- spinor accessors
+// How a field is read: LdNc through the read-only path (fields no running kernel writes), LdCg from
+// L2 (fields that other blocks of the same kernel write between grid barriers).
+struct LdNc {
+  template <class T>
+  __device__ __forceinline__ static T ld(const T* p) { return __ldg(p); }
+};
+struct LdCg {
+  template <class T>
+  __device__ __forceinline__ static T ld(const T* p) { return __ldcg(p); }
+};
+
 // Each spinor accessor holds one base pointer per parity (p0 even, p1 odd), so a
 // full field is two halves and a single-parity field leaves the other null.
 // FP64: [12][Vh] double2 per parity
@@ -335,13 +346,14 @@ struct SpinorF64 {
 };
 
 // FP32: [6][Vh] float4 per parity
-struct SpinorF32 {
+template <class Ld>
+struct SpinorF32T {
   float4* p0;
   float4* p1;
   int Vh;
   size_t rs = 0;
-  __device__ __forceinline__ SpinorF32 shift(int r) const {
-    SpinorF32 o = *this;
+  __device__ __forceinline__ SpinorF32T shift(int r) const {
+    SpinorF32T o = *this;
     if (p0) o.p0 = p0 + rs * r;
     if (p1) o.p1 = p1 + rs * r;
     return o;
@@ -351,7 +363,7 @@ struct SpinorF32 {
     Spinor<float> s;
 #pragma unroll
     for (int q = 0; q < 6; q++) {
-      float4 f = __ldg(b + q * Vh);
+      float4 f = Ld::ld(b + q * Vh);
       s.c[(2 * q) / 3][(2 * q) % 3] = {f.x, f.y};
       s.c[(2 * q + 1) / 3][(2 * q + 1) % 3] = {f.z, f.w};
     }
@@ -371,10 +383,12 @@ struct SpinorF32 {
     }
   }
 };
+using SpinorF32 = SpinorF32T<LdNc>;
 
 // FP16 with a per-site FP32 scale: [3][Vh] uint4 (8 halves each) + norm [Vh] per parity.
 // Stored value = component / norm, norm = max |real or imaginary part| over the site.
-struct SpinorF16 {
+template <class Ld>
+struct SpinorF16T {
   uint4* p0;
   uint4* p1;
   float* n0;
@@ -382,8 +396,8 @@ struct SpinorF16 {
   int Vh;
   size_t rs = 0;   // uint4 words between right-hand sides
   size_t rsn = 0;  // norms between right-hand sides
-  __device__ __forceinline__ SpinorF16 shift(int r) const {
-    SpinorF16 o = *this;
+  __device__ __forceinline__ SpinorF16T shift(int r) const {
+    SpinorF16T o = *this;
     if (p0) o.p0 = p0 + rs * r;
     if (p1) o.p1 = p1 + rs * r;
     if (n0) o.n0 = n0 + rsn * r;
@@ -392,11 +406,11 @@ struct SpinorF16 {
   }
   __device__ __forceinline__ Spinor<float> load(int parity, int cb) const {
     const uint4* b = (parity ? p1 : p0) + cb;
-    float n = __ldg((parity ? n1 : n0) + cb);
+    float n = Ld::ld((parity ? n1 : n0) + cb);
     Spinor<float> s;
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-      uint4 w = __ldg(b + q * Vh);
+      uint4 w = Ld::ld(b + q * Vh);
       uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int k = 0; k < 4; k++) {
@@ -413,11 +427,11 @@ struct SpinorF16 {
   static constexpr bool has_norm = true;
   __device__ __forceinline__ Spinor<float> load_raw(int parity, int cb, float& n) const {
     const uint4* b = (parity ? p1 : p0) + cb;
-    n = __ldg((parity ? n1 : n0) + cb);
+    n = Ld::ld((parity ? n1 : n0) + cb);
     Spinor<float> s;
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-      uint4 w = __ldg(b + q * Vh);
+      uint4 w = Ld::ld(b + q * Vh);
       uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int k = 0; k < 4; k++) {
@@ -451,6 +465,7 @@ struct SpinorF16 {
     (parity ? n1 : n0)[cb] = m;
   }
 };
+using SpinorF16 = SpinorF16T<LdNc>;
 
 // ---------------------------------------------------------------- link accessors
 // FP64 18-real: [parity][4][9][Vh] double2
