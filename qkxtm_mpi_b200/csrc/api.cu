@@ -115,17 +115,15 @@ int ensure_work(qkx_ctx* c) {
 
 // ---------------------------------------------------------------- reductions
 int finalize(qkx_ctx* c, int nparts, int mode, double* dst, int rhs) {
-  k_finalize<<<1, 1024, 0, c->st>>>(c->part, nparts, dst, mode, c->sc, rhs);
+  QKX_CUDA(launch_pdl(c, k_finalize, 1, 1024, c->part, nparts, dst, mode, c->sc, rhs));
   counted(c);
-  QKX_CUDA(cudaGetLastError());
   return QKX_OK;
 }
 
 int redot(qkx_ctx* c, const double2* x, const double2* y, size_t n, int mode, double* dst, int rhs) {
   int g = blas_grid(n);
-  k_redot<<<g, BLAS_NT, 0, c->st>>>(x, y, n, c->part);
+  QKX_CUDA(launch_pdl(c, k_redot, g, BLAS_NT, x, y, n, c->part));
   counted(c);
-  QKX_CUDA(cudaGetLastError());
   return finalize(c, g, mode, dst, rhs);
 }
 
@@ -834,10 +832,10 @@ int qkx_spinor_download(qkx_ctx* c, const double* dev, double* host) {
 int qkx_reCdotXdagY(qkx_ctx* c, const double* x, const double* y, double* result) {
   if (!c || !x || !y || !result) return invalid("NULL argument");
   QKX_CUDA(cudaSetDevice(c->device));
-  QKX_TRY(redot(c, (const double2*)x, (const double2*)y, 12 * c->V, FIN_STORE, c->dscal, 0));
-  QKX_CUDA(cudaMemcpyAsync(c->hscal, c->dscal, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  // the sum goes straight to page-locked host memory (no copy behind it)
+  QKX_TRY(redot(c, (const double2*)x, (const double2*)y, 12 * c->V, FIN_STORE, c->hscal, 0));
   QKX_CUDA(cudaStreamSynchronize(c->st));
-  *result = c->hscal[0];
+  *result = *(volatile double*)c->hscal;
   return QKX_OK;
 }
 
@@ -847,9 +845,8 @@ int qkx_X_eq_X_p_aY(qkx_ctx* c, double* x, double a, const double* y) {
   if (!c || !x || !y) return invalid("NULL argument");
   QKX_CUDA(cudaSetDevice(c->device));
   size_t n = 12 * c->V;
-  k_axpy_h<<<blas_grid(n), BLAS_NT, 0, c->st>>>(a, (const double2*)y, (double2*)x, n);
+  QKX_CUDA(launch_pdl(c, k_axpy_h, blas_grid(n), BLAS_NT, a, (const double2*)y, (double2*)x, n));
   counted(c);
-  QKX_CUDA(cudaGetLastError());
   return QKX_OK;
 }
 
@@ -857,9 +854,8 @@ int qkx_X_eq_aX_p_Y(qkx_ctx* c, double* x, double a, const double* y) {
   if (!c || !x || !y) return invalid("NULL argument");
   QKX_CUDA(cudaSetDevice(c->device));
   size_t n = 12 * c->V;
-  k_xpay_h<<<blas_grid(n), BLAS_NT, 0, c->st>>>((const double2*)y, a, (double2*)x, n);
+  QKX_CUDA(launch_pdl(c, k_xpay_h, blas_grid(n), BLAS_NT, (const double2*)y, a, (double2*)x, n));
   counted(c);
-  QKX_CUDA(cudaGetLastError());
   return QKX_OK;
 }
 

@@ -48,6 +48,7 @@ __device__ __forceinline__ double block_sum(double v) {
 // Re <x, y> over n complex numbers (partials per block)
 static __global__ void __launch_bounds__(BLAS_NT) k_redot(const double2* __restrict__ x, const double2* __restrict__ y,
                                                    size_t n, double* __restrict__ part) {
+  pdl_start();
   double acc = 0.0;
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
     double2 a = x[i], b = y[i];
@@ -63,6 +64,7 @@ enum { FIN_STORE = 0, FIN_PAP = 1, FIN_R2 = 2, FIN_R2_INIT = 3 };
 // Sum part[0..n) in a fixed order: FIN_STORE *dst = sum; FIN_R2_INIT r2 = sum
 static __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ part, int n, double* dst,
                                                    int mode, CgScalars* sc, int rhs) {
+  pdl_start();
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += 1024) acc += part[i];
   double s = block_sum<1024>(acc);
@@ -130,6 +132,7 @@ static __global__ void __launch_bounds__(BLAS_NT) k_cg_update(const CgScalars* s
 // y = y + a x with a host scalar
 static __global__ void __launch_bounds__(BLAS_NT) k_axpy_h(double a, const double2* __restrict__ x,
                                                     double2* __restrict__ y, size_t n) {
+  pdl_start();
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
     double2 xv = x[i], yv = y[i];
     y[i] = make_double2(yv.x + a * xv.x, yv.y + a * xv.y);
@@ -139,6 +142,7 @@ static __global__ void __launch_bounds__(BLAS_NT) k_axpy_h(double a, const doubl
 // y = a y + x with a host scalar
 static __global__ void __launch_bounds__(BLAS_NT) k_xpay_h(const double2* __restrict__ x, double a,
                                                     double2* __restrict__ y, size_t n) {
+  pdl_start();
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
     double2 xv = x[i], yv = y[i];
     y[i] = make_double2(a * yv.x + xv.x, a * yv.y + xv.y);

@@ -29,7 +29,9 @@
 // Tried and slower: 96 registers and 20 warps (0.158 ms for the 24^3x48 tm, 2.68 ms
 // for the batch), 80 registers with spills, both halves of a site in adjacent lanes
 // (0.156 ms, 2.78 ms), 128 sites a block, links past L1 (0.55 ms at 32^3x64), and L2
-// prefetches of the blocks to come (0.55-0.66 ms).
+// prefetches of the blocks to come (0.55-0.66 ms).  A pair of warps per direction on lattices that do not
+// fill the GPU is faster alone on it (8^3x16: 15.1 against 19.7 us for tm_xxDagTm_xx) and slower when
+// several lattices' calls overlap (12x14x10x18, three in flight: 21.7 against 15.0 us).
 //
 // NR right-hand sides per thread share the loaded link.  A block covers 32 sites
 // (two warps, one per s), so that s is uniform in a warp and the last wave is fine.
