@@ -425,6 +425,8 @@ def hop_link_bytes(precision, tile):
 
 def hop_kernel_name(precision, tile):
     """The sloppy hop kernel a tile (rhs_per_thread, threads_per_block, kind) launches."""
+    if tile[2] == 12:
+        return "hop_mu4_kernel"
     if 1 <= tile[2] <= 3:
         return "hop_pair_pf_kernel"
     if tile[2] == 10:

@@ -697,8 +697,8 @@ __global__ void __launch_bounds__(MAX_RHS) k_ctl_final(CgScalars* sc, MxCtl* ctl
 // context's stream while it is being captured (-1: top level, before anything else of the
 // branch; 0: top level before the outer loop; 4: top level after it; 1: outer body before the
 // inner loop; 2: outer body after it; 3: inner body; 5: the inner loop as one kernel, when
-// `inner_kernel`).  The kernels each level launched come back in *kt, *ko, *ki.  Both handles default to 0 at every launch, so a loop whose condition is never
-// set does not run.
+// `inner_kernel`).  The kernels each level launched come back in *kt, *ko, *ki.  Both handles
+// default to 0 at every launch, so a loop whose condition is never set does not run.
 template <class Emit>
 static int build_loop_graph(qkx_ctx* c, cudaGraph_t top, bool inner_kernel, long long* kt, long long* ko,
                             long long* ki, Emit emit) {
@@ -1206,6 +1206,7 @@ static bool small_batch(const qkx_ctx* c, int R_) { return mrhs_site_blocks<MU4_
 // rule.  On lattices from 6^3x12 to 32^3x64 and batches of 1 to 12 these were the tuner's choice or within
 // 3% of it (12 right-hand sides at 32^3x64: FP16 0.737 ms a hop with (2, 64, 11) against 1.07 with (1, 64, 0);
 // FP32 1.165 with (1, 64, 0) against 1.208 with (2, 128, 0)), so a first solve does not time tiles.
+// FP32 pairs on the packed pipe: 12 right-hand sides 1.067 ms, but 24^3x48 with 3 of them 0.127 against 0.105 ms.
 // alone: the solve has the GPU to itself (the branches of a batch of lattices have not, and run kernel by kernel).
 template <class P>
 static int tile_for(qkx_ctx* c, int R_, HopTile* tile, bool alone = true) {
