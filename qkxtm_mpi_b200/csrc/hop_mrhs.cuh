@@ -12,8 +12,9 @@
 // applyTwistAddDslash :1420 / applyTwistInv :1588 fused); one output parity.
 //
 // Grid: blockIdx.x = site_block * ngroups + group, group g covering the
-// right-hand sides [g*NR, g*NR + NR) of the batch.  (NR, NT) are chosen per
-// lattice and batch by the autotuner (tune_tile in mixed.cu).
+// right-hand sides [g*NR, g*NR + NR) of the batch.  (NR, NT) are chosen by rule
+// (tile_for in mixed.cu).  FP32 with one right-hand side a thread has its own kernel
+// (hop_f32.cuh).
 #pragma once
 #include <type_traits>
 
@@ -79,6 +80,60 @@ __device__ __forceinline__ void hop_dir_m(const SP (&in)[NR], const GA& gauge, c
   }
 }
 
+// The epilogue of one site and right-hand side from its hopping term acc; returns |o|^2 (of the CG residual for
+// EPI_XPAY_G5_CGR), or zero where no norm is asked for.
+template <typename R, int B, int EPI, class ARGS>
+__device__ __forceinline__ double mrhs_epilogue(const ARGS& A, int r, int par, int cb, const Spinor<R>& acc) {
+  const R a = R(A.a);
+  const R c = R(A.c * (A.cvec ? A.cvec[r] : 1.0));
+  const R sc = R(A.s * (A.svec ? A.svec[r] : 1.0));
+  double nrm = 0.0;
+  Spinor<R> o;
+  if constexpr (EPI == EPI_PLAIN) {
+    o = acc;
+  } else if constexpr (EPI == EPI_XPAY || EPI == EPI_XPAY_G5 || EPI == EPI_XPAY_G5_CGR) {
+    const Spinor<R> v = A.x.shift(r).load(par, cb);
+    const Spinor<R> g5v = gamma5<B>(v);
+#pragma unroll
+    for (int k = 0; k < 12; k++)
+      o.c[k / 3][k % 3] = a * acc.c[k / 3][k % 3] + (v.c[k / 3][k % 3] + c * phase<1>(g5v.c[k / 3][k % 3]));
+    if constexpr (EPI != EPI_XPAY) o = gamma5<B>(o);
+  } else if constexpr (EPI == EPI_TWIST_INV) {
+    o = twist_inv<B>(acc, c, sc);
+  } else {  // EPI_XPAY_TWINV
+    Spinor<R> v = A.x.shift(r).load(par, cb);
+#pragma unroll
+    for (int k = 0; k < 12; k++) v.c[k / 3][k % 3] = a * acc.c[k / 3][k % 3] + v.c[k / 3][k % 3];
+    o = twist_inv<B>(v, c, sc);
+  }
+  if constexpr (EPI == EPI_XPAY_G5_CGR) {
+    // the CG residual takes A p directly: r -= alpha A p, |r|^2 in FP64
+    const R al = R(A.alpha[r]);
+    auto rr = [&]() {
+      if constexpr (std::is_same<R, double>::value) return A.racc64.shift(r);
+      else return A.racc32.shift(r);
+    }();
+    Spinor<R> v = rr.load(par, cb);
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      Cx<R>& q = v.c[k / 3][k % 3];
+      q.re = q.re - al * o.c[k / 3][k % 3].re;
+      q.im = q.im - al * o.c[k / 3][k % 3].im;
+      nrm += double(q.re) * double(q.re) + double(q.im) * double(q.im);
+    }
+    rr.store(par, cb, v);
+  } else {
+    A.out.shift(r).store(par, cb, o);
+    if (A.norm_part) {
+#pragma unroll
+      for (int k = 0; k < 12; k++)
+        nrm += double(o.c[k / 3][k % 3].re) * double(o.c[k / 3][k % 3].re) +
+               double(o.c[k / 3][k % 3].im) * double(o.c[k / 3][k % 3].im);
+    }
+  }
+  return nrm;
+}
+
 // The work of one block: site block blk, group grp of NR right-hand sides.
 template <int NT, int NR, typename R, int B, bool DAG, int EPI, class ARGS>
 __device__ __forceinline__ void hop_mrhs_block(const ARGS& A, int blk, int grp) {
@@ -118,57 +173,9 @@ __device__ __forceinline__ void hop_mrhs_block(const ARGS& A, int blk, int grp) 
     hop_dir_m<NR, SP, GA, R, B, DAG, 2>(in, A.gauge, A.g, par, cb, x, s, L01, act, acc);
     hop_dir_m<NR, SP, GA, R, B, DAG, 3>(in, A.gauge, A.g, par, cb, x, s, L012, act, acc);
 
-    const R a = R(A.a);
 #pragma unroll
-    for (int j = 0; j < NR; j++) {
-      if (!act[j]) continue;
-      const int r = r0 + j;
-      const R c = R(A.c * (A.cvec ? A.cvec[r] : 1.0));
-      const R sc = R(A.s * (A.svec ? A.svec[r] : 1.0));
-      Spinor<R> o;
-      if constexpr (EPI == EPI_PLAIN) {
-        o = acc[j];
-      } else if constexpr (EPI == EPI_XPAY || EPI == EPI_XPAY_G5 || EPI == EPI_XPAY_G5_CGR) {
-        const Spinor<R> v = A.x.shift(r).load(par, cb);
-        const Spinor<R> g5v = gamma5<B>(v);
-#pragma unroll
-        for (int k = 0; k < 12; k++)
-          o.c[k / 3][k % 3] = a * acc[j].c[k / 3][k % 3] + (v.c[k / 3][k % 3] + c * phase<1>(g5v.c[k / 3][k % 3]));
-        if constexpr (EPI != EPI_XPAY) o = gamma5<B>(o);
-      } else if constexpr (EPI == EPI_TWIST_INV) {
-        o = twist_inv<B>(acc[j], c, sc);
-      } else {  // EPI_XPAY_TWINV
-        Spinor<R> v = A.x.shift(r).load(par, cb);
-#pragma unroll
-        for (int k = 0; k < 12; k++) v.c[k / 3][k % 3] = a * acc[j].c[k / 3][k % 3] + v.c[k / 3][k % 3];
-        o = twist_inv<B>(v, c, sc);
-      }
-      if constexpr (EPI == EPI_XPAY_G5_CGR) {
-        // the CG residual takes A p directly: r -= alpha A p, |r|^2 in FP64
-        const R al = R(A.alpha[r]);
-        auto rr = [&]() {
-          if constexpr (std::is_same<R, double>::value) return A.racc64.shift(r);
-          else return A.racc32.shift(r);
-        }();
-        Spinor<R> v = rr.load(par, cb);
-#pragma unroll
-        for (int k = 0; k < 12; k++) {
-          Cx<R>& q = v.c[k / 3][k % 3];
-          q.re = q.re - al * o.c[k / 3][k % 3].re;
-          q.im = q.im - al * o.c[k / 3][k % 3].im;
-          nrm[j] += double(q.re) * double(q.re) + double(q.im) * double(q.im);
-        }
-        rr.store(par, cb, v);
-      } else {
-        A.out.shift(r).store(par, cb, o);
-        if (A.norm_part) {
-#pragma unroll
-          for (int k = 0; k < 12; k++)
-            nrm[j] += double(o.c[k / 3][k % 3].re) * double(o.c[k / 3][k % 3].re) +
-                      double(o.c[k / 3][k % 3].im) * double(o.c[k / 3][k % 3].im);
-        }
-      }
-    }
+    for (int j = 0; j < NR; j++)
+      if (act[j]) nrm[j] = mrhs_epilogue<R, B, EPI>(A, r0 + j, par, cb, acc[j]);
   }
   if (A.norm_part) block_partials<NR, NT>(nrm, A.norm_part, A.nblk, r0, A.nrhs, blk);
 }

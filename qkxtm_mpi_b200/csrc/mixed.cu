@@ -39,6 +39,7 @@
 #include "hop.cuh"
 #include "hop_mrhs.cuh"
 #include "hop_mu4.cuh"
+#include "hop_f32.cuh"
 #include "hop_pair.cuh"
 #include "hop_c3t.cuh"
 #include "qkx_ctx.cuh"
@@ -968,6 +969,8 @@ static int launch_mrhs(qkx_ctx* c, int R_, const GA& gauge, const Geom& g, SP in
     hop_pair_as_kernel<NT, S, MINB, 0, false, EPI><<<A.nblk * ngrp, NT, 0, c->st>>>(A);
   } else if constexpr (f16 && NR % 2 == 0) {
     hop_pair_kernel<NT, NR / 2, 0, false, EPI><<<A.nblk * ngrp, NT, 0, c->st>>>(A);
+  } else if constexpr (NR == 1 && std::is_same<SP, SpinorF32>::value && std::is_same<GA, GaugeF32x12>::value) {
+    hop_f32_kernel<NT, 0, false, EPI><<<A.nblk * R_, NT, 0, c->st>>>(A);
   } else {
     hop_mrhs_kernel<NT, NR, SP, GA, R, 0, false, EPI><<<A.nblk * ngrp, NT, 0, c->st>>>(A);
   }
@@ -1205,8 +1208,8 @@ static bool small_batch(const qkx_ctx* c, int R_) { return mrhs_site_blocks<MU4_
 // The tile of a solve: the one qkx_tune or qkx_set_tile recorded for this precision and batch size, else by
 // rule.  On lattices from 6^3x12 to 32^3x64 and batches of 1 to 12 these were the tuner's choice or within
 // 3% of it (12 right-hand sides at 32^3x64: FP16 0.737 ms a hop with (2, 64, 11) against 1.07 with (1, 64, 0);
-// FP32 1.165 with (1, 64, 0) against 1.208 with (2, 128, 0)), so a first solve does not time tiles.
-// FP32 pairs on the packed pipe: 12 right-hand sides 1.067 ms, but 24^3x48 with 3 of them 0.127 against 0.105 ms.
+// FP32 1.057 with (1, 64, 0) against 1.206 with (2, 128, 0)), so a first solve does not time tiles.
+// FP32 pairs on the packed pipe: 12 right-hand sides 1.067 ms, 24^3x48 with 3 of them 0.127 against 0.094 ms.
 // alone: the solve has the GPU to itself (the branches of a batch of lattices have not, and run kernel by kernel).
 template <class P>
 static int tile_for(qkx_ctx* c, int R_, HopTile* tile, bool alone = true) {

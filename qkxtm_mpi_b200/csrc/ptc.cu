@@ -10,7 +10,7 @@
 #include <vector>
 
 #include "hop_c3t.cuh"
-#include "hop_mrhs.cuh"
+#include "hop_f32.cuh"
 #include "layout.cuh"
 #include "ptc.cuh"
 #include "ptc_tc.cuh"
@@ -503,7 +503,7 @@ static int hop32(qkx_ctx* c, int R, float4* in, int in_par, float4* out, float4*
   A.svec = svec;
   A.active = active;
   A.norm_part = nullptr;
-  hop_mrhs_kernel<64, 1, SpinorF32, GaugeF32x12, float, 0, false, EPI><<<A.nblk * R, 64, 0, c->st>>>(A);
+  hop_f32_kernel<64, 0, false, EPI><<<A.nblk * R, 64, 0, c->st>>>(A);
   counted(c);
   QKX_CUDA(cudaGetLastError());
   return QKX_OK;

@@ -59,3 +59,25 @@ def test_device_loop_and_host_loop_agree_bitwise(qkx, oracle, L, n, prec):
         assert e.value.code == qkx.ERR_NOT_CONVERGED
         last, _ = lat.invert(bs, precision=p, tol=1e-10)
         assert all(np.array_equal(x, y) for x, y in zip(xs, last))
+
+
+@pytest.mark.parametrize("L,n", [((2, 2, 2, 2), 1), ((6, 4, 2, 10), 3), ((8, 8, 8, 16), 5)])
+@pytest.mark.parametrize("nt", [64, 128, 256])
+def test_fp32_one_rhs_a_thread(qkx, oracle, L, n, nt):
+    """The FP32 hop that loads a term ahead: extents of 2 (both neighbours are one site), partial blocks, and
+    a solve in which one right-hand side is masked from the start."""
+    kappa, mu = 0.16, 0.01
+    U = oracle.apply_bc(L, oracle.gauge_random(L, 0.3, 91), -1)
+    bs = [oracle.spinor_gaussian(L, 92 + i) for i in range(n)]
+    with qkx.Lattice(qkx.LatticeInfo(L=L, kappa=kappa, mu=mu)) as lat:
+        lat.load_gauge(U)
+        for b, g in zip(bs, lat.sloppy_normal(bs, qkx.PREC_SINGLE, (1, nt, 0))):
+            assert rel(g, oracle.apply("tm_xx_dagtm_xx_ee", L, U, b, kappa, mu)) < 1e-5
+        if n == 1:
+            return
+        lat.set_tile(qkx.PREC_SINGLE, n, (1, nt, 0))
+        bs[0] = np.zeros_like(bs[0])
+        xs, _ = lat.invert(bs, precision=qkx.PREC_SINGLE, tol=1e-10)
+        assert not np.any(xs[0])
+        for b, x in zip(bs[1:], xs[1:]):
+            assert _res(oracle, L, U, x, b, kappa, mu) <= 1e-10
