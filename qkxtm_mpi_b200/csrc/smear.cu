@@ -117,22 +117,33 @@ int ape_run(qkx_ctx* c, const double2* in, double2* R, double2* T, int nsmear, d
 }
 
 // ---------------------------------------------------------------- Gaussian smearing
+// Up to this many blocks the steps overlap their launches: a step of 4^3x8 or 8x6x10x12 fields is as long as its
+// launch (10 steps of 12 fields on 4x6x4x8: 85 -> 76 us; 20 of 5 on 8x6x10x12: 206 -> 187), and 4,096 blocks
+// (16^3x32, 3 fields) still gain 4%.  At 62,208 (24^3x48, 12 fields) the wait costs 0.8%.
+constexpr unsigned GAUSS_PDL_BLOCKS = 8192;
+
 template <int NSP, int NR>
-void launch_gauss_t(qkx_ctx* c, const FieldPtrs& in, const FieldPtrs& out, int nrhs, int cb0, int ncb, double alpha,
-                    double norm) {
+int launch_gauss_t(qkx_ctx* c, const FieldPtrs& in, const FieldPtrs& out, int nrhs, int cb0, int ncb, double alpha,
+                   double norm) {
   const int nblk = (ncb + 31) / 32;
   const int ngrp = (nrhs + NR - 1) / NR;
-  k_gauss_step<NSP, NR><<<(unsigned)nblk * 2 * ngrp, 32 * 4 / NSP, 0, c->st>>>(in, out, GaugeF64x18{c->Usm, c->Vh},
-                                                                              c->geom, nrhs, cb0, ncb, alpha, norm);
+  const unsigned grid = (unsigned)nblk * 2 * ngrp, nt = 32 * 4 / NSP;
+  const GaugeF64x18 u{c->Usm, c->Vh};
+  if (grid <= GAUSS_PDL_BLOCKS)
+    QKX_CUDA(launch_pdl(c, k_gauss_step<NSP, NR, true>, grid, nt, in, out, u, c->geom, nrhs, cb0, ncb, alpha, norm));
+  else
+    k_gauss_step<NSP, NR, false><<<grid, nt, 0, c->st>>>(in, out, u, c->geom, nrhs, cb0, ncb, alpha, norm);
+  return QKX_OK;
 }
 
 // Four colour vectors a loaded link is the best use of the registers (times at the kernel): one spin of 4
 // fields, or of 3 where that leaves fewer spare slots (3, 5, 6, 9 fields), or two spins of 1 field for 1 or 2.
 int launch_gauss(qkx_ctx* c, const FieldPtrs& in, const FieldPtrs& out, int nrhs, int cb0, int ncb, double alpha,
                  double norm) {
-  if (nrhs <= 2) launch_gauss_t<2, 1>(c, in, out, nrhs, cb0, ncb, alpha, norm);
-  else if ((nrhs + 2) / 3 * 3 - nrhs < (nrhs + 3) / 4 * 4 - nrhs) launch_gauss_t<1, 3>(c, in, out, nrhs, cb0, ncb, alpha, norm);
-  else launch_gauss_t<1, 4>(c, in, out, nrhs, cb0, ncb, alpha, norm);
+  if (nrhs <= 2) QKX_TRY((launch_gauss_t<2, 1>(c, in, out, nrhs, cb0, ncb, alpha, norm)));
+  else if ((nrhs + 2) / 3 * 3 - nrhs < (nrhs + 3) / 4 * 4 - nrhs)
+    QKX_TRY((launch_gauss_t<1, 3>(c, in, out, nrhs, cb0, ncb, alpha, norm)));
+  else QKX_TRY((launch_gauss_t<1, 4>(c, in, out, nrhs, cb0, ncb, alpha, norm)));
   counted(c);
   QKX_CUDA(cudaGetLastError());
   return QKX_OK;

@@ -326,10 +326,12 @@ __device__ __forceinline__ void link_vec_acc(const Cd (&u)[9], const Cd (&v)[3],
 //   24^3x48,  1 field  (NSP 2, NR 1)   0.137 -> 0.120 ms      8x6x10x12, 5 fields        10.4 -> 8-10 us
 // Slower at 12 fields: (1, 1) 1.73, (1, 2) 1.36, (1, 3) 1.15, (1, 6) 1.21, (2, 1) 1.19, (2, 2) 1.21, (2, 3) 1.14 ms,
 // and 168 registers at 12 warps for any of them.
-template <int NSP, int NR>
+// PDL: launched with launch_pdl (the wait costs large steps 0.8%, so they are compiled without it).
+template <int NSP, int NR, bool PDL>
 __global__ void __launch_bounds__(32 * 4 / NSP, 4 * NSP)
     k_gauss_step(FieldPtrs in, FieldPtrs out, GaugeF64x18 u, Geom g, int nrhs, int cb0, int ncb, double alpha,
                  double norm) {
+  if constexpr (PDL) pdl_start();
   const int ngrp = (nrhs + NR - 1) / NR;
   const int r0 = (blockIdx.x % ngrp) * NR;
   const int bp = blockIdx.x / ngrp;

@@ -213,3 +213,20 @@ def test_gaussian_field_groups_and_partial_blocks(qkx, oracle, L, n):
         outs = lat.Gaussian_smearing(psis, nsmear=2, alpha=1.5)
     for p, o in zip(psis, outs):
         assert rel(o, oracle.gaussian_smear(L, U, p, 2, 1.5)) < 1e-13
+
+
+def test_gauss_steps_back_to_back(qkx, oracle):
+    """Steps whose launches overlap read what the step before wrote: many steps of a small batch, twice over, and
+    into a field that the next call reads."""
+    L = (4, 6, 2, 4)
+    U = oracle.gauge_random(L, 0.3, 7)
+    psi = oracle.spinor_gaussian(L, 8)
+    with qkx.Lattice(qkx.LatticeInfo(L=L, kappa=0.16, mu=0.01)) as lat:
+        lat.load_smearing_gauge(U)
+        a, b, c = lat.field(psi), lat.field(), lat.field()
+        for _ in range(2):
+            lat.Gaussian_smearing_dev([a], [b], nsmear=25, alpha=4.0)
+            lat.Gaussian_smearing_dev([b], [c], nsmear=24, alpha=4.0)
+        want = oracle.gaussian_smear(L, U, psi, 49, 4.0)
+        got = c.download()
+        assert rel(got, want) < 1e-13  # 49 steps of at most 1e-15 each
