@@ -46,8 +46,8 @@ __device__ __forceinline__ double block_sum(double v) {
 }
 
 // Re <x, y> over n complex numbers (partials per block)
-static __global__ void __launch_bounds__(BLAS_NT) k_redot(const double2* __restrict__ x, const double2* __restrict__ y,
-                                                   size_t n, double* __restrict__ part) {
+static __global__ void __launch_bounds__(BLAS_NT) k_redot(const double2* x, const double2* y, size_t n,
+                                                   double* part) {
   pdl_start();
   double acc = 0.0;
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
@@ -62,8 +62,8 @@ static __global__ void __launch_bounds__(BLAS_NT) k_redot(const double2* __restr
 enum { FIN_STORE = 0, FIN_PAP = 1, FIN_R2 = 2, FIN_R2_INIT = 3 };
 
 // Sum part[0..n) in a fixed order: FIN_STORE *dst = sum; FIN_R2_INIT r2 = sum
-static __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ part, int n, double* dst,
-                                                   int mode, CgScalars* sc, int rhs) {
+static __global__ void __launch_bounds__(1024) k_finalize(const double* part, int n, double* dst, int mode,
+                                                   CgScalars* sc, int rhs) {
   pdl_start();
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += 1024) acc += part[i];
@@ -87,7 +87,7 @@ static __global__ void k_cg_begin(CgScalars* sc, double stop) {
 
 // FIN_PAP: <p, M^+M p> = |M p|^2 from the first hop, alpha; FIN_R2: |r|^2 from the second, beta, the
 // stopping rule, and r2 to page-locked host memory
-static __global__ void __launch_bounds__(1024) k_cg_finalize(const double* __restrict__ part, int n, int mode,
+static __global__ void __launch_bounds__(1024) k_cg_finalize(const double* part, int n, int mode,
                                                       CgScalars* sc, double* r2_host) {
   pdl_start();
   if (mode == FIN_PAP) {
@@ -117,8 +117,8 @@ static __global__ void __launch_bounds__(1024) k_cg_finalize(const double* __res
 }
 
 // x = x + alpha p, p = r + beta p in one pass (X_eq_X_p_aY and X_eq_aX_p_Y, lib/blas_qkxTM.cpp:31, 45)
-static __global__ void __launch_bounds__(BLAS_NT) k_cg_update(const CgScalars* sc, const double2* __restrict__ r,
-                                                       double2* __restrict__ x, double2* __restrict__ p, size_t n) {
+static __global__ void __launch_bounds__(BLAS_NT) k_cg_update(const CgScalars* sc, const double2* r, double2* x,
+                                                       double2* p, size_t n) {
   pdl_start();
   if (!sc->restart[0]) return;
   const double a = sc->alpha[0], b = sc->beta[0];
@@ -130,8 +130,7 @@ static __global__ void __launch_bounds__(BLAS_NT) k_cg_update(const CgScalars* s
 }
 
 // y = y + a x with a host scalar
-static __global__ void __launch_bounds__(BLAS_NT) k_axpy_h(double a, const double2* __restrict__ x,
-                                                    double2* __restrict__ y, size_t n) {
+static __global__ void __launch_bounds__(BLAS_NT) k_axpy_h(double a, const double2* x, double2* y, size_t n) {
   pdl_start();
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
     double2 xv = x[i], yv = y[i];
@@ -140,8 +139,7 @@ static __global__ void __launch_bounds__(BLAS_NT) k_axpy_h(double a, const doubl
 }
 
 // y = a y + x with a host scalar
-static __global__ void __launch_bounds__(BLAS_NT) k_xpay_h(const double2* __restrict__ x, double a,
-                                                    double2* __restrict__ y, size_t n) {
+static __global__ void __launch_bounds__(BLAS_NT) k_xpay_h(const double2* x, double a, double2* y, size_t n) {
   pdl_start();
   for (size_t i = (size_t)blockIdx.x * BLAS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * BLAS_NT) {
     double2 xv = x[i], yv = y[i];

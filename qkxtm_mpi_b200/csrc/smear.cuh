@@ -366,34 +366,32 @@ __global__ void __launch_bounds__(32 * 4 / NSP, 4 * NSP)
       const double2* ul = d ? u.p + ((size_t)(1 - par) * 4 + mu) * 9 * Vh + nb : u.p + ((size_t)par * 4 + mu) * 9 * Vh + cb;
       Cd w[9];
 #pragma unroll
-      for (int k = 0; k < 9; k++) {
-        const double2 e = __ldg(ul + (size_t)k * Vh);
-        w[k] = {e.x, e.y};
-      }
+      for (int k = 0; k < 9; k++) w[k] = ld_link(ul + (size_t)k * Vh);
 #pragma unroll
       for (int j = 0; j < NR; j++)
 #pragma unroll
         for (int k = 0; k < NSP; k++) {
           Cd v[3];
 #pragma unroll
-          for (int a = 0; a < 3; a++) {
-            const double2 e = __ldg(f[j] + ((size_t)(1 - par) * 12 + k * 3 + a) * Vh + (d ? nb : nf));
-            v[a] = {e.x, e.y};
-          }
+          for (int a = 0; a < 3; a++) v[a] = ld_field(f[j] + ((size_t)(1 - par) * 12 + k * 3 + a) * Vh + (d ? nb : nf));
           if (d) link_vec_acc<true>(w, v, acc[j][k]);
           else link_vec_acc<false>(w, v, acc[j][k]);
         }
     }
   }
+  // the site's own words, all before the first store (a load cannot pass a store that might alias it)
+#pragma unroll
+  for (int j = 0; j < NR; j++)
+#pragma unroll
+    for (int k = 0; k < 3 * NSP; k++)
+      acc[j][k / 3][k % 3] = fma_s(alpha, acc[j][k / 3][k % 3], ld_field(f[j] + ((size_t)par * 12 + k) * Vh + cb));
 #pragma unroll
   for (int j = 0; j < NR; j++) {
     if (r0 + j >= nrhs) break;
     double2* o = const_cast<double2*>(out.p[r0 + j]) + ((size_t)par * 12 + s0 * 3) * Vh + cb;
-    const double2* own = f[j] + (size_t)par * 12 * Vh + cb;
 #pragma unroll
     for (int k = 0; k < 3 * NSP; k++) {
-      const double2 e = __ldg(own + (size_t)k * Vh);
-      const Cd t = fma_s(alpha, acc[j][k / 3][k % 3], Cd{e.x, e.y});
+      const Cd t = acc[j][k / 3][k % 3];
       o[(size_t)k * Vh] = make_double2(norm * t.re, norm * t.im);
     }
   }
