@@ -136,11 +136,15 @@ int launch_gauss_t(qkx_ctx* c, const FieldPtrs& in, const FieldPtrs& out, int nr
   return QKX_OK;
 }
 
-// Four colour vectors a loaded link is the best use of the registers (times at the kernel): one spin of 4
-// fields, or of 3 where that leaves fewer spare slots (3, 5, 6, 9 fields), or two spins of 1 field for 1 or 2.
+// Fields a thread (times at the kernel): six where they leave no spare slot and their blocks fill the SMs at three
+// each (148 * 3; below that, half as many blocks a field is the worse side: 12 fields on 4x6x4x8 9.2 us a step
+// against 9.0), else four or three, whichever leaves fewer spare slots, or two spins of one field for 1 or 2.
 int launch_gauss(qkx_ctx* c, const FieldPtrs& in, const FieldPtrs& out, int nrhs, int cb0, int ncb, double alpha,
                  double norm) {
+  const int pairs = (ncb + 31) / 32 * 2;  // blocks of 32 sites of both parities, for each group of fields
   if (nrhs <= 2) QKX_TRY((launch_gauss_t<2, 1>(c, in, out, nrhs, cb0, ncb, alpha, norm)));
+  else if (nrhs % 6 == 0 && (long long)pairs * (nrhs / 6) >= 148 * 3)
+    QKX_TRY((launch_gauss_t<1, 6>(c, in, out, nrhs, cb0, ncb, alpha, norm)));
   else if ((nrhs + 2) / 3 * 3 - nrhs < (nrhs + 3) / 4 * 4 - nrhs)
     QKX_TRY((launch_gauss_t<1, 3>(c, in, out, nrhs, cb0, ncb, alpha, norm)));
   else QKX_TRY((launch_gauss_t<1, 4>(c, in, out, nrhs, cb0, ncb, alpha, norm)));

@@ -297,19 +297,26 @@ struct FieldPtrs {
   const double2* p[MAX_RHS];
 };
 
-// acc += U v (DAG false) or U^+ v (DAG true) on one spin, in FMA chains
+// acc += U v (DAG false) or U^+ v (DAG true) on one spin; acc = U v for the first direction.  The three products of
+// a component are summed in one FMA chain and then added, so that the large running sum is rounded once a
+// direction.  Error of a step against the exact sum: 1.14e-16; one addition a product 1.32e-16, one FMA chain over
+// all 18 products 1.67e-16 (36 roundings at the size of the sum; 3-10% faster: 12 fields on 24^3x48 1.12 against
+// 1.16 ms a step, 4 fields 0.356 against 0.393).
 template <bool DAG>
-__device__ __forceinline__ void link_vec_acc(const Cd (&u)[9], const Cd (&v)[3], Cd (&acc)[3]) {
+__device__ __forceinline__ void link_vec_acc(const Cd (&u)[9], const Cd (&v)[3], Cd (&acc)[3], bool first) {
+  Cd t[3];
 #pragma unroll
-  for (int a = 0; a < 3; a++)
+  for (int b = 0; b < 3; b++)
 #pragma unroll
-    for (int b = 0; b < 3; b++) {
+    for (int a = 0; a < 3; a++) {
       const Cd e = DAG ? conj(u[b * 3 + a]) : u[a * 3 + b];
-      acc[a].re = fma(e.re, v[b].re, acc[a].re);
-      acc[a].im = fma(e.re, v[b].im, acc[a].im);
-      acc[a].re = fma(-e.im, v[b].im, acc[a].re);
-      acc[a].im = fma(e.im, v[b].re, acc[a].im);
+      t[a].re = b == 0 ? e.re * v[b].re : fma(e.re, v[b].re, t[a].re);
+      t[a].im = b == 0 ? e.re * v[b].im : fma(e.re, v[b].im, t[a].im);
+      t[a].re = fma(-e.im, v[b].im, t[a].re);
+      t[a].im = fma(e.im, v[b].re, t[a].im);
     }
+#pragma unroll
+  for (int a = 0; a < 3; a++) acc[a] = first ? t[a] : acc[a] + t[a];
 }
 
 // One smearing iteration on sites cb in [cb0, cb0 + ncb) of both parities:
@@ -322,13 +329,14 @@ __device__ __forceinline__ void link_vec_acc(const Cd (&u)[9], const Cd (&v)[3],
 //
 // What bounds it: the L1 data path (65% busy) and the latency of the gathers at 16 warps an SM; the FP64 pipe
 // is 38% busy.  Per step on one B200, against a whole site and two fields a thread (255 registers, 8 warps):
-//   24^3x48, 12 fields (NSP 1, NR 4)   1.29 -> 1.11 ms        16^3x32, 3 fields (1, 3)   0.074 -> 0.064 ms
-//   24^3x48,  1 field  (NSP 2, NR 1)   0.137 -> 0.120 ms      8x6x10x12, 5 fields        10.4 -> 8-10 us
-// Slower at 12 fields: (1, 1) 1.73, (1, 2) 1.36, (1, 3) 1.15, (1, 6) 1.21, (2, 1) 1.19, (2, 2) 1.21, (2, 3) 1.14 ms,
-// and 168 registers at 12 warps for any of them.
+//   24^3x48, 12 fields (NSP 1, NR 6)   1.33 -> 1.16 ms        16^3x32, 3 fields (1, 3)   0.074 -> 0.062 ms
+//   24^3x48,  4 fields (NSP 1, NR 4)   0.446 -> 0.393 ms      16^3x32, 12 fields (1, 6)  0.253 -> 0.205 ms
+//   24^3x48,  1 field  (NSP 2, NR 1)   0.134 -> 0.128 ms      8x6x10x12, 5 fields        11.7 -> 9.7 us
+// NR 6 runs at 168 registers and 12 warps an SM, the others at 128 and 16.  Slower at 12 fields: (1, 4) and (1, 3)
+// 1.21 ms; at 12 warps (1, 4) 1.35 ms.
 // PDL: launched with launch_pdl (the wait costs large steps 0.8%, so they are compiled without it).
 template <int NSP, int NR, bool PDL>
-__global__ void __launch_bounds__(32 * 4 / NSP, 4 * NSP)
+__global__ void __launch_bounds__(32 * 4 / NSP, (NSP * NR > 4 ? 3 : 4) * NSP)
     k_gauss_step(FieldPtrs in, FieldPtrs out, GaugeF64x18 u, Geom g, int nrhs, int cb0, int ncb, double alpha,
                  double norm) {
   if constexpr (PDL) pdl_start();
@@ -350,12 +358,6 @@ __global__ void __launch_bounds__(32 * 4 / NSP, 4 * NSP)
   for (int j = 0; j < NR; j++) f[j] = in.p[min(r0 + j, nrhs - 1)] + (size_t)(s0 * 3) * Vh;
   Cd acc[NR][NSP][3];
 #pragma unroll
-  for (int j = 0; j < NR; j++)
-#pragma unroll
-    for (int k = 0; k < NSP; k++)
-#pragma unroll
-      for (int a = 0; a < 3; a++) acc[j][k][a] = {0.0, 0.0};
-#pragma unroll
   for (int mu = 0; mu < 3; mu++) {
     const int stride = mu == 0 ? 1 : (mu == 1 ? L0 : L01);
     const int Lm = g.L[mu];
@@ -374,8 +376,8 @@ __global__ void __launch_bounds__(32 * 4 / NSP, 4 * NSP)
           Cd v[3];
 #pragma unroll
           for (int a = 0; a < 3; a++) v[a] = ld_field(f[j] + ((size_t)(1 - par) * 12 + k * 3 + a) * Vh + (d ? nb : nf));
-          if (d) link_vec_acc<true>(w, v, acc[j][k]);
-          else link_vec_acc<false>(w, v, acc[j][k]);
+          if (d) link_vec_acc<true>(w, v, acc[j][k], false);
+          else link_vec_acc<false>(w, v, acc[j][k], mu == 0);
         }
     }
   }
