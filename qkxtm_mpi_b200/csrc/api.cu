@@ -655,6 +655,10 @@ int qkx_create(const qkx_params* p, int device, qkx_ctx** out) {
     // allows them; the direct kernel is the default, as it is the faster of the two on B200
     const char* v = getenv("QKX_FP64_TILED");
     c->c3t = (v && v[0] == '1') ? 1 : 0;
+    // QKX_INNER_WAIT_MS: how long a block of a small solve's one-kernel inner loop waits for the others before the
+    // solve goes over to separate kernels (2000; 0: not at all)
+    v = getenv("QKX_INNER_WAIT_MS");
+    if (v && v[0] >= '0' && v[0] <= '9') c->inner_wait_ns = (unsigned long long)(std::min(atof(v), 1e6) * 1e6);
   }
   if (rc == QKX_OK && (e = cudaEventCreate(&c->t0)) != cudaSuccess) fail(e, "event");
   if (rc == QKX_OK && (e = cudaEventCreate(&c->t1)) != cudaSuccess) fail(e, "event");

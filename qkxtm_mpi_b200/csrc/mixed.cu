@@ -353,6 +353,7 @@ struct MxCtl {
   int iter, since, n_ru, n_outer, n_restart, diverged;
   int nan_rhs, nan_iter;   // first right-hand side whose r^2 became NaN or inf, and when (0: none)
   int unconverged;         // right-hand sides still active when the loop ended
+  int gave_up;             // a grid barrier of the one-kernel inner loop ran out of time: the loop's results are void
   unsigned long long t_ru0, ru_ns;  // device clock at the start of the last update; summed update time
   double cv[MAX_RHS], sv[MAX_RHS];  // per-RHS twist factors, staged here (page-locked) for the set-up's copies
 };
@@ -452,20 +453,20 @@ struct InnerArgs {
   CgScalars* sc;
   MxCtl* ctl;
   unsigned long long* bar;  // arrivals at the grid barrier
-  int* err;       // the context's status word
+  unsigned long long wait_ns;  // longest wait there
 };
 
 constexpr int SMALL_ITEMS = 148 * 4;
-constexpr unsigned long long INNER_WAIT_NS = 2000000000ull;  // longest wait at a grid barrier
 
 // The blocks of a cooperative grid meet at a counter that only grows: each adds one (release) and thread 0 polls
 // (acquire) until everybody has.  Starts from the multiple of the grid size at or below the counter,
 // which fewer than gridDim.x blocks can have passed when a block begins.
 struct GridBarrier {
   unsigned long long* count;
-  unsigned long long target;
-  int* err;
-  __device__ __forceinline__ GridBarrier(unsigned long long* c, int* e) : count(c), target(0), err(e) {
+  unsigned long long target, wait_ns;
+  int* gave_up;
+  __device__ __forceinline__ GridBarrier(unsigned long long* c, unsigned long long w, int* g)
+      : count(c), target(0), wait_ns(w), gave_up(g) {
     if (threadIdx.x == 0) {
       const unsigned long long v = peek();
       target = v - v % gridDim.x;
@@ -476,7 +477,8 @@ struct GridBarrier {
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
     return v;
   }
-  // false (and a code in *err) when a block does not arrive in time
+  // false (and *gave_up set) when a block does not arrive in time; with no time at all, when one is missing at the
+  // first look
   __device__ __forceinline__ bool meet() {
     __shared__ int ok;
     __syncthreads();
@@ -486,12 +488,13 @@ struct GridBarrier {
       int good = 1;
       unsigned polls = 0;
       unsigned long long t0 = 0;
+      const unsigned every = wait_ns ? 255u : 0u;  // looks at the clock every 256 polls
       while (peek() < target) {
-        if ((++polls & 255u) == 0) {
+        if ((++polls & every) == 0) {
           const unsigned long long t = mx_clock_ns();
           if (t0 == 0) t0 = t;
-          if (t - t0 > INNER_WAIT_NS) {
-            atomicCAS(err, 0, 2);
+          if (t - t0 >= wait_ns) {
+            atomicExch(gave_up, 1);
             good = 0;
             break;
           }
@@ -532,10 +535,15 @@ __global__ void __launch_bounds__(128) k_inner_small(InnerArgs<SP, AC, GA> A) {
     active[i] = A.sc->active[i];
     alpha[i] = beta[i] = 0.0;
   }
-  GridBarrier grid(A.bar, A.err);
+  GridBarrier grid(A.bar, A.wait_ns, &A.ctl->gave_up);
   int iter = A.ctl->iter, since = A.ctl->since;
   const int maxIter = A.ctl->maxIter;
+  if (tid == 0) bad = A.ctl->gave_up;
   __syncthreads();
+  if (bad) {  // an earlier pass of this solve gave up: its arrivals are still in the counter
+    if (first) A.ctl->iter = maxIter;
+    return;
+  }
   HopArgs<SP, GA, AC> H;
   H.gauge = A.U;
   H.g = A.g;
@@ -641,7 +649,7 @@ __global__ void __launch_bounds__(128) k_inner_small(InnerArgs<SP, AC, GA> A) {
     }
     if (!grid.meet()) break;
   }
-  if (first) A.ctl->iter = maxIter;  // a barrier gave up: no further pass (the status word voids the solve)
+  if (first) A.ctl->iter = maxIter;  // a barrier gave up: no further pass (invert_eo_mixed_t starts over without this kernel)
 }
 
 // after a reliable update (|rhat|^2 in aux, |Mh^+ rhat|^2 in aux2): converged and diverged RHS
@@ -1083,7 +1091,7 @@ struct Sloppy {
       A.sc = c->sc;
       A.ctl = m->ctl;
       A.bar = m->bar;
-      A.err = c->dstat;
+      A.wait_ns = c->inner_wait_ns;
       int per_sm = 0, sms = 0;
       QKX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_inner_small<SPC, ACC, GA, R>, 128, 0));
       QKX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
@@ -1315,6 +1323,7 @@ struct MixedSolve {
   dim3 cg2, bg2;
   bool device_loop = false;
   bool inner_kernel = false;  // the inner loop is one kernel
+  bool have_b = false;        // bE and bO hold the right-hand sides already
   long long kcount[3] = {};  // kernels of the loop graph's top level, outer pass and inner pass
   // results of the host-driven loop (the device loop keeps them in MxCtl)
   int iter = 0, n_ru = 0, n_restart = 0, diverged = 0, nact = 0;
@@ -1326,8 +1335,9 @@ struct MixedSolve {
       : c(c_), sp(sp_), nrhs(nrhs_), b(b_), x(x_), active(nrhs_, 1), bnorm2(nrhs_) {}
 
   // alone: nothing else is meant to run on the GPU beside this solve (a batch of lattices is not alone,
-  // and a cooperative kernel would wait for room for its whole grid)
-  int prepare(bool allow_device_loop, bool alone) {
+  // and a cooperative kernel would wait for room for its whole grid).  one_kernel: the inner loop of a small batch
+  // may be one kernel.
+  int prepare(bool allow_device_loop, bool alone, bool one_kernel = true) {
     QKX_TRY(mixed_alloc<P>(c, nrhs, true));
     m = c->mixed;
     QKX_TRY(tile_for<P>(c, nrhs, &tile, alone));
@@ -1344,7 +1354,7 @@ struct MixedSolve {
     // the whole iteration loop on the device (one graph launch) unless the hop kernels are being
     // timed one by one (event records cannot sit inside a conditional graph body) or graphs are off
     device_loop = allow_device_loop && sp->use_graphs != 0 && c->prof == 0;
-    inner_kernel = device_loop && alone && tile.kind == 12 && small_batch(c, nrhs);
+    inner_kernel = device_loop && alone && one_kernel && tile.kind == 12 && small_batch(c, nrhs);
     MxCtl* hc = m->ctl_h;
     memset(hc, 0, sizeof(MxCtl));
     hc->nrhs = nrhs;
@@ -1372,10 +1382,11 @@ struct MixedSolve {
     QKX_CUDA(cudaMemcpyAsync(c->sc, c->sc_h, sizeof(CgScalars), cudaMemcpyHostToDevice, c->st));
     if (device_loop) QKX_CUDA(cudaMemcpyAsync(m->ctl, hc, sizeof(MxCtl), cudaMemcpyHostToDevice, c->st));
     if (inner_kernel) QKX_CUDA(cudaMemsetAsync(m->bar, 0, sizeof(unsigned long long), c->st));
-    for (int i = 0; i < nrhs; i++) {
+    for (int i = 0; i < nrhs && !have_b; i++) {
       QKX_CUDA(cudaMemcpyAsync(m->bE + i * n12, b[i], hb, cudaMemcpyDeviceToDevice, c->st));
       QKX_CUDA(cudaMemcpyAsync(m->bO + i * n12, b[i] + n12, hb, cudaMemcpyDeviceToDevice, c->st));
     }
+    have_b = true;
     k_mx_norm<<<bg2, MX_NT, 0, c->st>>>(B64(m->bE, 0, Vh), m->part);
     counted(c);
     k_mx_finalize<<<nrhs, 256, 0, c->st>>>(m->part, MX_GRID, FIN_AUX, c->sc);
@@ -1743,6 +1754,12 @@ struct MixedSolve {
     return QKX_OK;
   }
 
+  // count the kernels that the loop graph launched (its scalars in host memory)
+  void count_loop() {
+    const MxCtl* hc = m->ctl_h;
+    counted(c, (int)(kcount[0] + (long long)hc->n_outer * kcount[1] + (long long)hc->iter * kcount[2]));
+  }
+
   // status and solve info once the final phase's copies are in host memory; rel (optional) gets
   // every RHS's true residual ||b - M x|| / ||b||.  Device times: the phase marks when given.
   int finish(qkx_solve_info* info, double* rel, const float* ms_total, const float* ms_setup, const float* ms_final) {
@@ -1756,7 +1773,7 @@ struct MixedSolve {
       nact = hc->unconverged;
       ms_ru = float(hc->ru_ns * 1e-6);
       for (int i = 0; i < nrhs; i++) bnorm2[i] = hc->bnorm2[i];
-      counted(c, (int)(kcount[0] + (long long)hc->n_outer * kcount[1] + (long long)hc->iter * kcount[2]));
+      count_loop();
       if (hc->nan_iter > 0) {
         set_error("mixed CG: r2 of right-hand side %d became non-finite at iteration %d", hc->nan_rhs, hc->nan_iter);
         return QKX_ERR_NAN;
@@ -1801,17 +1818,25 @@ static int invert_eo_mixed_t(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, 
   QKX_TRY(s.prepare(true, true));
   MixedState* m = c->mixed;
   QKX_CUDA(cudaEventRecord(c->t0, c->st));
-  QKX_TRY(s.setup());
-  QKX_CUDA(cudaEventRecord(m->ph[0], c->st));  // set-up done
-  if (s.device_loop) {
-    QKX_TRY(s.device_loop_launch());
-  } else {
-    QKX_TRY(s.host_loop());
+  for (;;) {
+    QKX_TRY(s.setup());
+    QKX_CUDA(cudaEventRecord(m->ph[0], c->st));  // set-up done
+    if (s.device_loop) {
+      QKX_TRY(s.device_loop_launch());
+    } else {
+      QKX_TRY(s.host_loop());
+    }
+    QKX_CUDA(cudaEventRecord(m->ph[3], c->st));  // the final phase starts where the loop ended
+    QKX_TRY(s.final_phase());
+    QKX_CUDA(cudaEventRecord(c->t1, c->st));
+    QKX_CUDA(cudaEventSynchronize(c->t1));
+    if (!s.inner_kernel || !m->ctl_h->gave_up) break;
+    // A block of the one-kernel inner loop waited too long for the others (the GPU was taken away from it): the
+    // same solve again, kernel by kernel, which waits for nothing.  bE and bO still hold the right-hand sides;
+    // the caller's may have been overwritten (a solution may take its source's place).
+    s.count_loop();
+    QKX_TRY(s.prepare(true, true, false));
   }
-  QKX_CUDA(cudaEventRecord(m->ph[3], c->st));  // the final phase starts where the loop ended
-  QKX_TRY(s.final_phase());
-  QKX_CUDA(cudaEventRecord(c->t1, c->st));
-  QKX_CUDA(cudaEventSynchronize(c->t1));
   float ms = 0, ms_setup = 0, ms_final = 0;
   cudaEventElapsedTime(&ms, c->t0, c->t1);
   cudaEventElapsedTime(&ms_setup, c->t0, m->ph[0]);

@@ -69,6 +69,8 @@ struct qkx_ctx {
   qkx::CgScalars* sc_h = nullptr;  // pinned host mirror
   double* dscal = nullptr;         // device scratch scalars [64]
   double* hscal = nullptr;         // pinned host scalars [64]
+  // longest wait of a block at a barrier of the one-kernel inner loop (QKX_INNER_WAIT_MS at creation)
+  unsigned long long inner_wait_ns = 2000000000ull;
   int* dstat = nullptr;            // device status word: non-zero after a bounded device wait gave up
   int* hstat = nullptr;            // pinned host copy
   int smem_optin = 0;              // shared memory a block may opt in to on this device

@@ -1,0 +1,79 @@
+"""The mixed solver's inner loop as one cooperative kernel: which batches take it (at most 592 items of 32 sites and
+one right-hand side, alone on the GPU), several blocks an SM, masked right-hand sides, its barrier's limit,
+and solves beside each other.  A solve whose iterations are launched kernel by kernel counts more than eight launches
+an iteration; with one kernel for the inner loop it counts only those around it."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+KAPPA, MU, TOL = 0.16, 0.01, 1e-10
+
+
+def _lattice(qkx, oracle, L, seed=81):
+    U = oracle.apply_bc(L, oracle.gauge_random(L, 0.3, seed), -1)
+    lat = qkx.Lattice(qkx.LatticeInfo(L=L, kappa=KAPPA, mu=MU))
+    lat.load_gauge(U)
+    return lat, U
+
+
+def _res(O, L, U, x, b):
+    return float(np.linalg.norm(b - O.apply("tm", L, U, x, KAPPA, MU)) / np.linalg.norm(b))
+
+
+def _solve(lat, bs, **kw):
+    k = lat.kernel_launches()
+    xs, info = lat.invert(bs, tol=TOL, **kw)
+    return xs, info, lat.kernel_launches() - k
+
+
+def _one_kernel(info, launches):
+    return launches < 4 * info.iterations
+
+
+# items: 297, 384, 473, 512, 592 (the last that the rule takes), 594
+@pytest.mark.parametrize("prec", ["half", "single"])
+@pytest.mark.parametrize("L,n,inside", [((22, 6, 12, 12), 1, True), ((8, 8, 8, 16), 3, True),
+                                        ((12, 14, 10, 18), 1, True), ((8, 8, 8, 16), 4, True),
+                                        ((4, 4, 8, 74), 4, True), ((22, 6, 12, 12), 2, False)])
+def test_rule_and_host_loop_bits(qkx, oracle, L, n, inside, prec):
+    p = {"half": qkx.PREC_HALF, "single": qkx.PREC_SINGLE}[prec]
+    lat, U = _lattice(qkx, oracle, L)
+    with lat:
+        bs = [oracle.spinor_gaussian(L, 82 + i) for i in range(n)]
+        if n > 2:
+            bs[1] = np.zeros_like(bs[1])  # masked from the start
+        xs, info, k = _solve(lat, bs, precision=p)
+        assert _one_kernel(info, k) == inside
+        host, ih, kh = _solve(lat, bs, precision=p, use_graphs=0)
+        assert not _one_kernel(ih, kh)
+        assert (info.iterations, info.reliable_updates, info.restarts) == (ih.iterations, ih.reliable_updates, ih.restarts)
+        for b, x, y in zip(bs, xs, host):
+            assert np.array_equal(x, y)
+            assert _res(oracle, L, U, x, b) <= TOL if np.any(b) else not np.any(x)
+
+
+@pytest.mark.parametrize("L,n", [((8, 8, 8, 16), 1), ((8, 8, 8, 16), 3)])
+@pytest.mark.parametrize("prec", ["half", "single"])
+def test_barrier_that_gives_up_leaves_the_solve_to_the_kernels(qkx, oracle, monkeypatch, L, n, prec):
+    """With no time to wait the blocks give up at their first barrier; the solve then runs kernel by kernel
+    from the start and has the bits of the host-driven loop, again and again on the same context, the
+    solution field being the source's own as well."""
+    p = {"half": qkx.PREC_HALF, "single": qkx.PREC_SINGLE}[prec]
+    monkeypatch.setenv("QKX_INNER_WAIT_MS", "0")
+    lat, U = _lattice(qkx, oracle, L)
+    monkeypatch.delenv("QKX_INNER_WAIT_MS")
+    with lat:
+        bs = [oracle.spinor_gaussian(L, 82 + i) for i in range(n)]
+        host, ih, _ = _solve(lat, bs, precision=p, use_graphs=0)
+        for _ in range(2):
+            xs, info, k = _solve(lat, bs, precision=p)
+            assert info.converged == 1 and info.iterations == ih.iterations and not _one_kernel(info, k)
+            for b, x, y in zip(bs, xs, host):
+                assert np.array_equal(x, y) and _res(oracle, L, U, x, b) <= TOL
+        f = [lat.field(b) for b in bs]
+        assert lat.invert_dev(f, f, precision=p, tol=TOL).converged == 1
+        for q, y in zip(f, host):
+            assert np.array_equal(q.download(), y)
+            q.close()
