@@ -1059,8 +1059,10 @@ static int invert_cg_fp64(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, con
   return worst;
 }
 
-int qkx_invert_dev(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double* const* b_dev,
-                   double* const* x_dev, qkx_solve_info* info) {
+}  // extern "C"
+
+int qkx::invert_dev(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double* const* b_dev,
+                    double* const* x_dev, qkx_solve_info* info, bool alone) {
   if (!c || !sp || !b_dev || !x_dev) return invalid("NULL argument");
   if (nrhs < 1 || nrhs > MAX_RHS) return invalid("nrhs must be in 1..64");
   for (int i = 0; i < nrhs; i++)
@@ -1076,11 +1078,18 @@ int qkx_invert_dev(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const doub
   double2* const* x = (double2* const*)x_dev;
   int rc;
   if (sp->method == QKX_SOLVER_CG_FP64) rc = invert_cg_fp64(c, sp, nrhs, b, x, info);
-  else if (sp->method == QKX_SOLVER_CG_EO_MIXED) rc = invert_eo_mixed(c, sp, nrhs, b, x, info);
-  else if (sp->method == QKX_SOLVER_GCR_PTC) rc = invert_gcr_ptc(c, sp, nrhs, b, x, info);
+  else if (sp->method == QKX_SOLVER_CG_EO_MIXED) rc = invert_eo_mixed(c, sp, nrhs, b, x, info, alone);
+  else if (sp->method == QKX_SOLVER_GCR_PTC) rc = invert_gcr_ptc(c, sp, nrhs, b, x, info, alone);
   else return invalid("solver method");
   const int st = device_status(c);  // a bounded device wait that gave up voids the solution
   return st != QKX_OK ? st : rc;
+}
+
+extern "C" {
+
+int qkx_invert_dev(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double* const* b_dev,
+                   double* const* x_dev, qkx_solve_info* info) {
+  return invert_dev(c, sp, nrhs, b_dev, x_dev, info, true);
 }
 
 int qkx_invert(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double* const* b_host,

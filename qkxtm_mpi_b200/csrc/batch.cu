@@ -51,6 +51,7 @@ int qkx_invert_batch(qkx_batch_job* jobs, int njobs, const qkx_solver_params* sp
       }
     return QKX_OK;
   }
+  const bool alone = ctxs.size() == 1;
   std::vector<std::thread> threads;
   for (qkx_ctx* c : ctxs) {
     threads.emplace_back([=]() {
@@ -58,7 +59,8 @@ int qkx_invert_batch(qkx_batch_job* jobs, int njobs, const qkx_solver_params* sp
         if (jobs[i].ctx != c) continue;
         qkx_solver_params p = *sp;
         p.mu = jobs[i].mu;
-        jobs[i].status = qkx_invert_dev(c, &p, jobs[i].nrhs, jobs[i].b_dev, jobs[i].x_dev, &jobs[i].info);
+        // with other lattices' threads beside it no solve counts as alone on the GPU, as in the one-graph path
+        jobs[i].status = invert_dev(c, &p, jobs[i].nrhs, jobs[i].b_dev, jobs[i].x_dev, &jobs[i].info, alone);
         jobs[i].message[0] = 0;
         if (jobs[i].status != QKX_OK) {  // the message is per thread: keep it in the job
           snprintf(jobs[i].message, sizeof jobs[i].message, "%s", qkx_last_error());

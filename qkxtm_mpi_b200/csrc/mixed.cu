@@ -1813,9 +1813,9 @@ struct MixedSolve {
 
 template <class P>
 static int invert_eo_mixed_t(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double2* const* b,
-                             double2* const* x, qkx_solve_info* info) {
+                             double2* const* x, qkx_solve_info* info, bool alone) {
   MixedSolve<P> s(c, sp, nrhs, b, x);
-  QKX_TRY(s.prepare(true, true));
+  QKX_TRY(s.prepare(true, alone));
   MixedState* m = c->mixed;
   QKX_CUDA(cudaEventRecord(c->t0, c->st));
   for (;;) {
@@ -1835,7 +1835,7 @@ static int invert_eo_mixed_t(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, 
     // same solve again, kernel by kernel, which waits for nothing.  bE and bO still hold the right-hand sides;
     // the caller's may have been overwritten (a solution may take its source's place).
     s.count_loop();
-    QKX_TRY(s.prepare(true, true, false));
+    QKX_TRY(s.prepare(true, alone, false));
   }
   float ms = 0, ms_setup = 0, ms_final = 0;
   cudaEventElapsedTime(&ms, c->t0, c->t1);
@@ -2177,15 +2177,15 @@ int tune(qkx_ctx* c, int precision, int nrhs, int* nr, int* nt, double* ms) {
 }
 
 int invert_eo_mixed(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double2* const* b, double2* const* x,
-                    qkx_solve_info* info) {
-  if (sp->sloppy_precision == QKX_PREC_DOUBLE) return invert_eo_mixed_t<PDouble>(c, sp, nrhs, b, x, info);
+                    qkx_solve_info* info, bool alone) {
+  if (sp->sloppy_precision == QKX_PREC_DOUBLE) return invert_eo_mixed_t<PDouble>(c, sp, nrhs, b, x, info, alone);
   if (!c->compressible) {
     set_error("mixed precision needs SU(3) links (12-real reconstruction); these links are not unitary "
               "to 1e-6 (max |UU^+-1| = %g)", c->link_unitarity);
     return QKX_ERR_UNSUPPORTED;
   }
-  if (sp->sloppy_precision == QKX_PREC_SINGLE) return invert_eo_mixed_t<PSingle>(c, sp, nrhs, b, x, info);
-  if (sp->sloppy_precision == QKX_PREC_HALF) return invert_eo_mixed_t<PHalf>(c, sp, nrhs, b, x, info);
+  if (sp->sloppy_precision == QKX_PREC_SINGLE) return invert_eo_mixed_t<PSingle>(c, sp, nrhs, b, x, info, alone);
+  if (sp->sloppy_precision == QKX_PREC_HALF) return invert_eo_mixed_t<PHalf>(c, sp, nrhs, b, x, info, alone);
   set_error("invalid argument: sloppy_precision");
   return QKX_ERR_INVALID;
 }

@@ -575,7 +575,7 @@ struct EoScratch {
 };
 
 int invert_gcr_ptc(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double2* const* b, double2* const* x,
-                   qkx_solve_info* info) {
+                   qkx_solve_info* info, bool alone) {
   QKX_TRY(check_ready(c));
   qkx_ptc* net = const_cast<qkx_ptc*>(sp->preconditioner);
   if (net && net->c != c) return bad("the preconditioner belongs to another context");
@@ -849,7 +849,7 @@ int invert_gcr_ptc(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const doub
     for (int i = 0; i < nF; i++) fmu[i] = mu[fbl[i]];
     fp.mu = fmu.data();
     qkx_solve_info fi{};
-    const int frc = invert_eo_mixed(c, &fp, nF, bb.data(), xx.data(), &fi);
+    const int frc = invert_eo_mixed(c, &fp, nF, bb.data(), xx.data(), &fi, alone);
     if (frc != QKX_OK && frc != QKX_ERR_NOT_CONVERGED) return frc;
     fb_iters = fi.iterations;
     for (int i = 0; i < nF; i++) {

@@ -171,16 +171,19 @@ inline SpinorF64 H64(const double2* base, int parity, int Vh) {
   return parity ? SpinorF64{nullptr, b, Vh} : SpinorF64{b, nullptr, Vh};
 }
 
-// mixed-precision solver entry (mixed.cu)
+// mixed-precision solver entry (mixed.cu); alone: no other solve is meant to run on the GPU beside this one
 int invert_eo_mixed(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double2* const* b,
-                    double2* const* x, qkx_solve_info* info);
+                    double2* const* x, qkx_solve_info* info, bool alone = true);
+// qkx_invert_dev; alone as above
+int invert_dev(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double* const* b_dev, double* const* x_dev,
+               qkx_solve_info* info, bool alone);
 void mixed_free(qkx_ctx* c);
 // qkx_invert_batch as one graph launch for all lattices (CG_EO_MIXED, graphs on): 0 done,
 // 1 not applicable, < 0 error; t0 is the batch's start on the steady clock, in seconds
 int invert_batch_graph(qkx_batch_job* jobs, int njobs, const qkx_solver_params* sp, double t0);
 // the learned solver: batched even-odd flexible CG preconditioned by the network (ptc.cu)
 int invert_gcr_ptc(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double2* const* b, double2* const* x,
-                   qkx_solve_info* info);
+                   qkx_solve_info* info, bool alone = true);
 void mixed_invalidate(qkx_ctx* c);
 int tune(qkx_ctx* c, int precision, int nrhs, int* nr, int* nt, double* ms);
 int set_tile(qkx_ctx* c, int precision, int nrhs, int nr, int nt, int kind);

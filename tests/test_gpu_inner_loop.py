@@ -77,3 +77,51 @@ def test_barrier_that_gives_up_leaves_the_solve_to_the_kernels(qkx, oracle, monk
         for q, y in zip(f, host):
             assert np.array_equal(q.download(), y)
             q.close()
+
+
+def test_two_solves_at_once(qkx, oracle):
+    """Two threads, two lattices, solve after solve: the cooperative grids take turns or share the GPU, and every
+    solution has the bits of the same solve alone."""
+    specs = [((8, 8, 8, 16), 4), ((12, 14, 10, 18), 1)]
+    lats = [_lattice(qkx, oracle, L, 90 + i) for i, (L, _) in enumerate(specs)]
+    bs = [[oracle.spinor_gaussian(L, 91 + 7 * i + r) for r in range(n)] for i, (L, n) in enumerate(specs)]
+    alone = [lat.invert(b, tol=TOL)[0] for (lat, _), b in zip(lats, bs)]
+    bad = []
+
+    def work(i):
+        try:
+            for _ in range(20):
+                xs, info = lats[i][0].invert(bs[i], tol=TOL)
+                if info.converged != 1 or not all(np.array_equal(x, y) for x, y in zip(xs, alone[i])):
+                    bad.append(i)
+        except Exception as e:  # noqa: BLE001
+            bad.append(e)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for lat, _ in lats:
+        lat.close()
+    assert not bad
+
+
+def test_a_batch_of_lattices_is_not_alone(qkx, oracle):
+    """invert_batch's path with a thread per lattice (here: one lattice's hops are being timed) takes no
+    cooperative loop either: its lattices share the GPU."""
+    specs = [((8, 8, 8, 16), 2), ((6, 4, 2, 10), 3)]
+    lats = [_lattice(qkx, oracle, L, 95 + i) for i, (L, _) in enumerate(specs)]
+    bs = [[oracle.spinor_gaussian(L, 96 + 7 * i + r) for r in range(n)] for i, (L, n) in enumerate(specs)]
+    jobs = [(lat, [lat.field(b) for b in v], [lat.field() for _ in v], [MU] * len(v)) for (lat, _), v in zip(lats, bs)]
+    lats[1][0].profile(True)
+    k = [lat.kernel_launches() for lat, _ in lats]
+    res = qkx.invert_batch(jobs, tol=TOL)
+    lats[1][0].profile(False)
+    for (lat, U), job, v, r, k0, (L, _) in zip(lats, jobs, bs, res, k, specs):
+        assert r["status"] == qkx.OK and lat.kernel_launches() - k0 > 4 * r["info"]["iterations"]
+        for x, b in zip(job[2], v):
+            assert _res(oracle, L, U, x.download(), b) <= TOL
+        for f in job[1] + job[2]:
+            f.close()
+        lat.close()
