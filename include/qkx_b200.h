@@ -292,7 +292,9 @@ QKX_API int qkx_invert_batch(qkx_batch_job* jobs, int njobs, const qkx_solver_pa
  * size: times every tile (right-hand sides per thread x threads per block x kind) on
  * the device and keeps the fastest for later solves.  A solve with an untuned
  * (precision, nrhs) takes its tile by a rule on the lattice, precision and batch
- * size.  No reference counterpart. */
+ * size; so does, tuned or not, a half or single solve of a batch that does not
+ * fill the GPU (kind 12 below), as its inner loop is then one kernel, which the
+ * times of single hops say nothing about.  No reference counterpart. */
 QKX_API int qkx_tune(qkx_ctx* ctx, int precision, int nrhs, int* rhs_per_thread, int* threads_per_block,
                      double* ms_per_hop);
 
@@ -311,9 +313,9 @@ QKX_API int qkx_tune(qkx_ctx* ctx, int precision, int nrhs, int* rhs_per_thread,
  * do not fill the GPU; a solve of such a batch alone on the GPU then runs its
  * inner iterations in one kernel.
  *
- * Use this tile (one of the tuner's) for later CG_EO_MIXED solves and
- * qkx_sloppy_normal calls with this precision and batch size, instead of the
- * tuned one.  No reference counterpart. */
+ * Use this tile (one that qkx_tune times, or kind 10) for later CG_EO_MIXED
+ * solves and qkx_sloppy_normal calls with this precision and batch size,
+ * instead of the tuned one or the rule's.  No reference counterpart. */
 QKX_API int qkx_set_tile(qkx_ctx* ctx, int precision, int nrhs, int rhs_per_thread, int threads_per_block,
                          int kind);
 
@@ -326,7 +328,8 @@ QKX_API int qkx_tune_table(qkx_ctx* ctx, int precision, int nrhs, int max, int* 
 /* out_r = Vector::tm_xxDagTm_xx(.., EE) in_r (lib/lattice_util.cpp:2024) for a
  * batch, computed the way one inner iteration of CG_EO_MIXED computes A p: the
  * even sites of in_r rounded to the sloppy precision, then the four sloppy hops
- * with the given tile (one of the tuner's; 0, 0, 0 = the tuned tile).  Odd sites of out_r are zero.  Host buffers in
+ * with the given tile (one that qkx_set_tile takes; 0, 0, 0 = the pinned or tuned
+ * tile, else the rule's).  Odd sites of out_r are zero.  Host buffers in
  * Vector::M layout.  A hook for checking every tile against the FP64 operator;
  * no reference counterpart. */
 QKX_API int qkx_sloppy_normal(qkx_ctx* ctx, int precision, int nrhs, int rhs_per_thread, int threads_per_block,

@@ -631,7 +631,7 @@ class Lattice:
 
     def set_tile(self, precision: int, nrhs: int, tile) -> None:
         """Use this hop tile (rhs_per_thread, threads_per_block[, kind]) for later mixed solves of
-        this precision and batch size instead of the tuned one."""
+        this precision and batch size instead of the tuned one or the rule's."""
         t = tuple(tile) + (0,) * (3 - len(tile))
         check(lib().qkx_set_tile(self.ctx, precision, nrhs, int(t[0]), int(t[1]), int(t[2])))
 
@@ -649,8 +649,8 @@ class Lattice:
     def sloppy_normal(self, psis: Sequence[np.ndarray], precision: int = PREC_HALF, tile=(0, 0, 0)) -> list:
         """tm_xxDagTm_xx(EE) of every field as the mixed solver's inner iteration computes it: the
         even sites rounded to the sloppy precision and the four sloppy hops with the given tile
-        (rhs_per_thread, threads_per_block[, kind]); (0, 0, 0) = the tuned tile.  Odd sites of the
-        results are zero."""
+        (rhs_per_thread, threads_per_block[, kind]); (0, 0, 0) = the pinned or tuned tile, else the
+        rule's.  Odd sites of the results are zero."""
         psis = [_host(p) for p in psis]
         outs = [np.zeros_like(p) for p in psis]
         n = len(psis)

@@ -1202,7 +1202,7 @@ static int tune_tile(qkx_ctx* c, int R_, HopTile* best, double* best_ms) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc == QKX_OK) {
-    c->tuned[P::id * 1000 + R_] = {best->nr, best->nt, best->kind};
+    c->tuned[P::id * 1000 + R_] = {best->nr, best->nt, best->kind, false};
     c->tune_log[P::id * 1000 + R_] = log;
   }
   return rc;
@@ -1213,17 +1213,20 @@ static int tune_tile(qkx_ctx* c, int R_, HopTile* best, double* best_ms) {
 // one) the two ways take the same time, and above that the tiles that fill the GPU win.
 static bool small_batch(const qkx_ctx* c, int R_) { return mrhs_site_blocks<MU4_NS>(c->Vh) * R_ <= SMALL_ITEMS; }
 
-// The tile of a solve: the one qkx_tune or qkx_set_tile recorded for this precision and batch size, else by
+// The tile of a solve: the one qkx_set_tile or qkx_tune recorded for this precision and batch size, else by
 // rule.  On lattices from 6^3x12 to 32^3x64 and batches of 1 to 12 these were the tuner's choice or within
 // 3% of it (12 right-hand sides at 32^3x64: FP16 0.737 ms a hop with (2, 64, 11) against 1.07 with (1, 64, 0);
 // FP32 1.057 with (1, 64, 0) against 1.206 with (2, 128, 0)), so a first solve does not time tiles.
 // FP32 pairs on the packed pipe: 12 right-hand sides 1.067 ms, 24^3x48 with 3 of them 0.127 against 0.094 ms.
 // alone: the solve has the GPU to itself (the branches of a batch of lattices have not, and run kernel by kernel).
+// whole_loop: the tile is for a solve.  The tuner times hops one by one and not the one-kernel inner loop, which is
+// faster on every small batch (8^3x16 with four right-hand sides, FP16: kind 9 and kind 12 both 7.9 us a hop), so
+// its choice yields to the rule there; a pinned tile does not.
 template <class P>
-static int tile_for(qkx_ctx* c, int R_, HopTile* tile, bool alone = true) {
+static int tile_for(qkx_ctx* c, int R_, HopTile* tile, bool alone = true, bool whole_loop = false) {
   auto it = c->tuned.find(P::id * 1000 + R_);
-  const bool small = alone && small_batch(c, R_);
-  if (it != c->tuned.end()) {
+  const bool small = alone && P::id != QKX_PREC_DOUBLE && small_batch(c, R_);
+  if (it != c->tuned.end() && (it->second.pinned || !(small && whole_loop))) {
     tile->nr = it->second.nr;
     tile->nt = it->second.nt;
     tile->kind = it->second.kind;
@@ -1340,7 +1343,7 @@ struct MixedSolve {
   int prepare(bool allow_device_loop, bool alone, bool one_kernel = true) {
     QKX_TRY(mixed_alloc<P>(c, nrhs, true));
     m = c->mixed;
-    QKX_TRY(tile_for<P>(c, nrhs, &tile, alone));
+    QKX_TRY(tile_for<P>(c, nrhs, &tile, alone, true));
     Vh = c->Vh;
     n12 = 12 * (size_t)Vh;
     hb = sizeof(double2) * n12;
@@ -2097,7 +2100,7 @@ int set_tile(qkx_ctx* c, int precision, int nrhs, int nr, int nt, int kind) {
     return QKX_ERR_INVALID;
   }
   if (!known_tile(precision, nr, nt, kind)) return QKX_ERR_INVALID;
-  c->tuned[precision * 1000 + nrhs] = {nr, nt, kind};
+  c->tuned[precision * 1000 + nrhs] = {nr, nt, kind, true};
   return QKX_OK;
 }
 

@@ -35,6 +35,7 @@ struct MixedState;
 
 struct qkx_tile_rec {
   int nr = 0, nt = 0, kind = 0;
+  bool pinned = false;  // by qkx_set_tile; else qkx_tune's choice
 };
 
 struct qkx_ctx {
@@ -90,7 +91,7 @@ struct qkx_ctx {
   long long kernels = 0;
   int capturing = 0;          // set while a CUDA graph is being captured
   long long captured = 0;     // kernels recorded into the graph being captured
-  // tuned tiles: (precision*1000 + nrhs) -> (RHS per thread, threads per block, kernel kind)
+  // tuned and pinned tiles: (precision*1000 + nrhs) -> (RHS per thread, threads per block, kernel kind)
   std::map<int, qkx_tile_rec> tuned;
   // every tile timed by the last tuning of a key: (nr, nt, kind, ms per hop)
   std::map<int, std::vector<std::array<double, 4>>> tune_log;

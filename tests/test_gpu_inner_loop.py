@@ -125,3 +125,26 @@ def test_a_batch_of_lattices_is_not_alone(qkx, oracle):
         for f in job[1] + job[2]:
             f.close()
         lat.close()
+
+
+@pytest.mark.parametrize("prec", ["half", "single"])
+@pytest.mark.parametrize("L,n", [((4, 4, 4, 8), 1), ((8, 8, 8, 16), 1), ((8, 8, 8, 16), 3), ((12, 14, 10, 18), 1),
+                                 ((8, 8, 8, 16), 4), ((22, 6, 12, 12), 1)])
+def test_tuning_keeps_the_one_kernel_loop(qkx, oracle, L, n, prec):
+    """qkx_tune times hops one by one: whichever tile it picks, a small batch alone on the GPU keeps its one-kernel
+    loop.  A tile set by hand is taken."""
+    p = {"half": qkx.PREC_HALF, "single": qkx.PREC_SINGLE}[prec]
+    lat, U = _lattice(qkx, oracle, L)
+    with lat:
+        bs = [oracle.spinor_gaussian(L, 82 + i) for i in range(n)]
+        xs, info, k = _solve(lat, bs, precision=p)
+        assert _one_kernel(info, k)
+        lat.tune(p, n)
+        again, it, kt = _solve(lat, bs, precision=p)
+        assert _one_kernel(it, kt) and all(np.array_equal(x, y) for x, y in zip(xs, again))
+        lat.set_tile(p, n, (1, 64, 0))
+        _, it, kt = _solve(lat, bs, precision=p)
+        assert not _one_kernel(it, kt)
+        lat.set_tile(p, n, (1, 128, 12))
+        again, it, kt = _solve(lat, bs, precision=p)
+        assert _one_kernel(it, kt) and all(np.array_equal(x, y) for x, y in zip(xs, again))
