@@ -902,8 +902,10 @@ static int cg_fp64_loop(qkx_ctx* c, double2* x, double2* r, double2* p, double2*
   counted(c);
   long long queued = 0, read = 0;
   const long long most = (long long)maxIter - *k;
+  // one at a time while the hops are timed: those of an iteration past the stop move nothing
+  const int ahead = c->prof ? 1 : qkx_ctx::CG_AHEAD;
   while (r2 > stop && read < most) {
-    while (queued < most && queued < read + qkx_ctx::CG_AHEAD) {
+    while (queued < most && queued < read + ahead) {
       QKX_TRY(cg_fp64_iteration(c, x, r, p, tmp, slot + queued % qkx_ctx::CG_AHEAD));
       QKX_CUDA(cudaEventRecord(c->cg_ev[queued % qkx_ctx::CG_AHEAD], c->st));
       queued++;
