@@ -444,8 +444,8 @@ int run_op(qkx_ctx* c, int op, const double2* in, double2* out) {
   const double k = c->p.kappa, mu = c->p.mu, s = c->p.twistSign;
   const double tw = 2.0 * k * mu * s;
   const double inv = 1.0 / (1.0 + (2.0 * k * mu) * (2.0 * k * mu));
-  double2* t1 = c->w[6];
-  double2* t2 = c->w[7];
+  double2* t1 = c->w[5];
+  double2* t2 = c->w[6];
   if (in == t1 || in == t2 || out == t1 || out == t2) return invalid("operator fields alias the work fields");
   switch (op) {
     case QKX_OP_DSLASH: return hop64(c, 0, false, EPI_PLAIN, in, out, nullptr, -1, 0, 0, 1);
@@ -944,10 +944,10 @@ int qkx_cg_dev(qkx_ctx* c, const double* in_dev, double* x_dev, qkx_solve_info* 
   }
   QKX_CUDA(cudaSetDevice(c->device));
   QKX_TRY(ensure_work(c));
-  double2 *r = c->w[2], *p = c->w[3], *tmp = c->w[5];
+  double2 *r = c->w[2], *p = c->w[3], *tmp = c->w[4];
   const double2* in = (const double2*)in_dev;
   double2* x = (double2*)x_dev;
-  for (double2* f : {r, p, c->w[4], tmp})
+  for (double2* f : {r, p, tmp})
     if ((const double2*)in == f || x == f) return invalid("CG fields alias the context's work fields");
   QKX_CUDA(cudaEventRecord(c->t0, c->st));
   double r2, src;
@@ -990,12 +990,12 @@ int qkx_cg(qkx_ctx* c, const double* in_host, double* x_host, qkx_solve_info* in
 }
 
 // ---------------------------------------------------------------- invert
-// ||b - M x||^2 and ||b||^2 in FP64 (uses w[6] for M x)
+// ||b - M x||^2 and ||b||^2 in FP64 (uses w[5] for M x)
 static int true_residual(qkx_ctx* c, const double2* b, const double2* x, double* rel) {
   const size_t n = 12 * c->V;
-  QKX_TRY(apply_tm(c, x, c->w[6], false));
+  QKX_TRY(apply_tm(c, x, c->w[5], false));
   int g = blas_grid(n);
-  k_sub_norm<<<g, BLAS_NT, 0, c->st>>>(b, c->w[6], c->w[6], n, c->part);
+  k_sub_norm<<<g, BLAS_NT, 0, c->st>>>(b, c->w[5], c->w[5], n, c->part);
   counted(c);
   QKX_CUDA(cudaGetLastError());
   QKX_TRY(finalize(c, g, FIN_STORE, c->dscal + 2, 0));
@@ -1012,12 +1012,11 @@ static int true_residual(qkx_ctx* c, const double2* b, const double2* x, double*
 static int invert_cg_fp64(qkx_ctx* c, const qkx_solver_params* sp, int nrhs, const double2* const* b,
                           double2* const* x, qkx_solve_info* info) {
   QKX_TRY(ensure_work(c));
-  double2 *in = c->w[0], *r = c->w[2], *p = c->w[3], *Ap = c->w[4], *tmp = c->w[5];
+  double2 *in = c->w[0], *r = c->w[2], *p = c->w[3], *tmp = c->w[4], *mx = c->w[5];
   const size_t n = 12 * c->V;
   for (int i = 0; i < nrhs; i++) {
-    if (b[i] == in || x[i] == in || b[i] == r || x[i] == r || b[i] == p || x[i] == p || b[i] == Ap ||
-        x[i] == Ap || b[i] == tmp || x[i] == tmp || b[i] == c->w[6] || x[i] == c->w[6])
-      return invalid("invert fields alias the context's work fields");
+    for (const double2* f : {in, r, p, tmp, mx})
+      if (b[i] == f || x[i] == f) return invalid("invert fields alias the context's work fields");
   }
   QKX_CUDA(cudaEventRecord(c->t0, c->st));
   int worst = QKX_OK;

@@ -62,8 +62,8 @@ struct qkx_ctx {
   double2* Usm = nullptr;     // [2][4][9][Vh] FP64 links of the Gaussian smearing (APE-smeared)
   int have_smear = 0;
   double2* stage = nullptr;   // one host-layout spinor (V*12 double2)
-  static constexpr int NW = 8;
-  double2* w[NW] = {};        // FP64 full-lattice work fields
+  static constexpr int NW = 7;
+  double2* w[NW] = {};        // FP64 full-lattice work fields: in, out; CG r, p, M p; two of operators and residuals
   double* part = nullptr;     // reduction partials
   int npart = 0;
   qkx::CgScalars* sc = nullptr;    // device solver scalars

@@ -1,5 +1,7 @@
 """The plain FP64 CG queues iterations ahead of the residual it reads: stops at maxIter, and what the profile of
 its hops counts."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -52,3 +54,28 @@ def test_profile_counts_the_hops_of_the_iterations_only(qkx, oracle, setup):
     V = b.size // 24
     # a hop reads the field and the links and writes a field; the second also reads the residual it updates
     assert by == info.iterations * V * (2 * (2 * 192.0 + 4 * 144.0) + 192.0)
+
+
+def test_work_fields_that_nothing_reads_are_not_held(qkx, oracle):
+    """An operator, a CG and a solve of 16^3 x 32 (24 MiB a field) hold seven work fields."""
+    import torch
+
+    def run(L):
+        lat = qkx.Lattice(qkx.LatticeInfo(L=L, kappa=KAPPA, mu=MU, maxIter=1000))
+        lat.generate_gauge(0.3, 5)
+        b, x = lat.field(oracle.spinor_gaussian(L, 55)), lat.field()
+        lat.sync()
+        free = torch.cuda.mem_get_info()[0]
+        lat.apply_dev("tm_xx_dagtm_xx_ee", b, x)
+        info = qkx.SolveInfo()
+        x.upload(np.zeros((lat.V, 4, 3, 2)))
+        qkx.check(qkx.lib().qkx_cg_dev(lat.ctx, b.ptr, x.ptr, C.byref(info)))
+        lat.invert_dev([b], [x], method=qkx.SOLVER_CG_FP64, tol=1e-8)
+        used = free - torch.cuda.mem_get_info()[0]
+        b.close(), x.close(), lat.close()
+        return used
+
+    run((4, 4, 4, 8))  # loads every kernel
+    L = (16, 16, 16, 32)
+    field = 16 * 16 * 16 * 32 * 192
+    assert run(L) < 7.5 * field
