@@ -114,3 +114,16 @@ def test_partial_site_blocks_and_momentum_chunks(qkx, oracle, L, Q):
         if Q < 9:
             for op in range(2):
                 assert _close(lat.delta_2pt(p1, p2, op, Q, xs), oracle.delta_2pt(L, p1, p2, op, Q, xs)), op
+
+
+@pytest.mark.parametrize("L,Q", [((2, 34, 2, 2), 2), ((2, 65, 2, 3), 5), ((4, 33, 2, 2), 0)])
+def test_more_rows_than_a_warp(qkx, oracle, L, Q):
+    """L_y = 33, 34 and 65: a warp of the transform takes its plane's rows in two and three turns and adds to
+    the sums of the turn before."""
+    p1, p2 = seeded_propagator(L, 21 + L[1]), seeded_propagator(L, 22 + L[1])
+    xs = (1, 5, 0, 0)
+    with qkx.Lattice(qkx.LatticeInfo(L=L)) as lat:
+        m = lat.meson_2pt(p1, [0, 3, 9], Q, xs)
+        for k, op in enumerate((0, 3, 9)):
+            assert _close(m[k], oracle.meson_2pt(L, p1, op, Q, xs)), op
+        assert _close(lat.baryon_2pt(p1, p2, 0, Q, xs), oracle.baryon_2pt(L, p1, p2, 0, Q, xs))
