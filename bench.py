@@ -437,6 +437,8 @@ def hop_kernel_name(precision, tile):
         return "hop_pair_as_kernel"
     if precision in ("half", "fp16") and tile[0] % 2 == 0:
         return "hop_pair_kernel"
+    if precision in ("single", "fp32") and tile[0] == 1:
+        return "hop_f32_kernel"
     return "hop_mrhs_kernel"
 
 
@@ -786,7 +788,7 @@ def main():
     ap.add_argument("--lattice", type=lambda v: tuple(int(x) for x in v.split(",")), default=L,
                     help="X,Y,Z,T for the non-default workloads")
     ap.add_argument("--tile", type=lambda v: tuple(int(x) for x in v.split(",")), default=None,
-                    help="RHS_PER_THREAD,THREADS_PER_BLOCK,KIND of the sloppy hop instead of the autotuner's")
+                    help="RHS_PER_THREAD,THREADS_PER_BLOCK,KIND of the sloppy hop instead of the one that lat.tune picks")
     args = ap.parse_args()
     if args.warmup < 3:
         print("note: --warmup below 3 raised to 3", file=sys.stderr)
