@@ -79,3 +79,20 @@ def test_work_fields_that_nothing_reads_are_not_held(qkx, oracle):
     L = (16, 16, 16, 32)
     field = 16 * 16 * 16 * 32 * 192
     assert run(L) < 7.5 * field
+
+
+def test_cg_on_the_tiled_hop(qkx, oracle, monkeypatch):
+    """QKX_FP64_TILED=1: the first hop of an iteration on TMA row tiles, with its norm and the mask of queued
+    iterations, the second on the direct kernel; same steps, FP64 rounding apart."""
+    L = (16, 8, 4, 8)
+    U = oracle.apply_bc(L, oracle.gauge_random(L, 0.3, 57), -1)
+    b = oracle.spinor_gaussian(L, 58)
+    out = []
+    for mode in ("0", "1"):
+        monkeypatch.setenv("QKX_FP64_TILED", mode)
+        with qkx.Lattice(qkx.LatticeInfo(L=L, kappa=KAPPA, mu=MU, tol=1e-10, maxIter=1000)) as lat:
+            lat.load_gauge(U)
+            out.append(lat.cg(b))
+    (x, i), (y, j) = out
+    assert i.converged == j.converged == 1 and i.iterations == j.iterations
+    assert rel(y, x) < 1e-9
