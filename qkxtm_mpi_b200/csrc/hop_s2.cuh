@@ -23,10 +23,11 @@
 // every projection three times (5.2 KB a site).  Measured on one B200:
 //                                              colour threads   this kernel
 //   tm, 32^3x64 (both parities, one launch)        0.600 ms       0.463 ms   (4.3 TB/s of algorithmic bytes)
-//   tm, 24^3x48                                    0.203 ms       0.152 ms
+//   tm, 24^3x48                                    0.199 ms       0.157 ms
 //   A^-1 D, one parity, 24^3x48                    0.122 ms       0.094 ms   (5.4 TB/s)
 //   A^-1 D, one parity, 32^3x64, 12 RHS            3.77 ms        2.36 ms    (NR = 2; 2.60 with NR = 1)
-// Tried and slower: 96 registers and 20 warps (0.158 ms for the 24^3x48 tm, 2.68 ms
+//   tm_xxDagTm_xx, 24^3x48 (four hops)             0.515 ms       0.400 ms
+// (the two one-parity times with the fields on the read-only path).  Tried and slower: 96 registers and 20 warps (0.158 ms for the 24^3x48 tm, 2.68 ms
 // for the batch), 80 registers with spills, both halves of a site in adjacent lanes
 // (0.156 ms, 2.78 ms), 128 sites a block, links past L1 (0.55 ms at 32^3x64), and L2
 // prefetches of the blocks to come (0.55-0.66 ms).  A pair of warps per direction on lattices that do not

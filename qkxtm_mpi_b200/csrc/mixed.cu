@@ -42,6 +42,7 @@
 #include "hop_f32.cuh"
 #include "hop_pair.cuh"
 #include "hop_c3t.cuh"
+#include "hop_s2.cuh"
 #include "qkx_ctx.cuh"
 #include "site_ops.cuh"
 
@@ -437,8 +438,8 @@ __global__ void __launch_bounds__(MAX_RHS) k_ctl_after_iter(const CgScalars* sc,
 // same numbers, so no scalar travels between kernels.  The hops are hop_mu4_block's and the update is
 // k_mx_update_p's, so the bits are those of the kernel-by-kernel loop with tile kind 12.
 // Fields that blocks exchange are read from L2 (LdCg).
-// 8^3x16, one source, FP16: 33 -> 20 us an iteration (five barriers of about 1.3 us), the solve of 32
-// iterations 1.60 -> 1.23 ms; three sources 1.69 -> 1.41; 6^3x12 1.51 -> 1.16; 12x14x10x18 1.71 -> 1.46 ms.
+// 8^3x16, one source, FP16: 35.5 -> 27.4 us an iteration (five barriers of about 1.3 us), the solve of 32
+// iterations 1.48 -> 1.21 ms; three sources 38.8 -> 31.1 us; 6^3x12 35.7 -> 25.2 us; 12x14x10x18 38.5 -> 33.8 us.
 // With a fence, an arrival counter and a generation word instead of one growing counter, 1.39 ms.
 template <class SP, class AC, class GA>
 struct InnerArgs {
@@ -857,10 +858,10 @@ static int mixed_alloc(qkx_ctx* c, int R, bool solver) {
     if (rc == QKX_OK && !f->d) rc = bfield_alloc<typename P::SP>(*f, m->R, Vh);
   if (rc == QKX_OK && !m->cvec && cudaMalloc(&m->cvec, sizeof(double) * MAX_RHS) != cudaSuccess) rc = QKX_ERR_NOMEM;
   if (rc == QKX_OK && !m->svec && cudaMalloc(&m->svec, sizeof(double) * MAX_RHS) != cudaSuccess) rc = QKX_ERR_NOMEM;
-  // partials: the smallest hop block (64 threads) or the FP64 hop's row tiles (whichever is more)
-  // over both parities, plus the streaming grid
+  // partials of a right-hand side, room for both parities: the smallest blocks are those of MU4_NS sites (the sloppy
+  // hops) and of S2_NS or the row tiles (the FP64 hop); plus the streaming grid
   const size_t nblk =
-      (size_t)std::max(hop_blocks_per_rhs<64>(Vh, -1), c3t_blocks(c->geom, -1)) + MX_GRID;
+      (size_t)std::max({2 * mrhs_site_blocks<MU4_NS>(Vh), s2_blocks_per_rhs(Vh, -1), c3t_blocks(c->geom, -1)}) + MX_GRID;
   if (rc == QKX_OK && !m->part && cudaMalloc(&m->part, sizeof(double) * (size_t)m->R * nblk) != cudaSuccess)
     rc = QKX_ERR_NOMEM;
   if (solver) {

@@ -327,8 +327,8 @@ __device__ __forceinline__ void link_vec_acc(const Cd (&u)[9], const Cd (&v)[3],
 // blockIdx.x = ((block * 2) + parity) * ngroups + group, the groups of one site block adjacent so
 // their shared links stay in L2.
 //
-// What bounds it: the L1 data path (65% busy) and the latency of the gathers at 16 warps an SM; the FP64 pipe
-// is 38% busy.  Per step on one B200, against a whole site and two fields a thread (255 registers, 8 warps):
+// What bounds it: the L1 data path (57% busy) and the latency of the gathers at 12 warps an SM; the FP64 pipe
+// is 44% busy, DRAM 39% (24^3x48, 12 fields).  Per step on one B200, against a whole site and two fields a thread (255 registers, 8 warps):
 //   24^3x48, 12 fields (NSP 1, NR 6)   1.33 -> 1.16 ms        16^3x32, 3 fields (1, 3)   0.074 -> 0.062 ms
 //   24^3x48,  4 fields (NSP 1, NR 4)   0.446 -> 0.393 ms      16^3x32, 12 fields (1, 6)  0.253 -> 0.205 ms
 //   24^3x48,  1 field  (NSP 2, NR 1)   0.134 -> 0.128 ms      8x6x10x12, 5 fields        11.7 -> 9.7 us
